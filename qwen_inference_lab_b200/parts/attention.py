@@ -47,7 +47,7 @@ import math
 
 import torch
 
-from ..kernels import attention_mma, gemm_tc, ops
+from ..kernels import attention_f32, attention_mma, gemm_tc, ops
 from .base import KVCacheSpec, Mixer, Param, StateSpec, StepPlanner
 from .linear import Linear, StackedLinear
 from .rotary import RotaryFrequencies
@@ -379,6 +379,10 @@ class GroupedQueryAttention(Mixer):
         if tensor_cores:
             attention_mma.attend(ctx, q, cache, out, self.n_q_heads, self.n_kv_heads, self.head_dim,
                                  self.window, self.scale, self._slopes_log2, v_dim=self.v_head_dim)
+            return
+        if self._slopes is None and attention_f32.supports(q, cache.pages, self.head_dim, self.v_head_dim, self.n_q_heads,
+                                                           self.n_kv_heads):
+            attention_f32.attend(ctx, q, cache, out, self.n_q_heads, self.n_kv_heads, self.head_dim, self.window, self.scale)
             return
         ops.attention_generic(q, cache.pages, out, ctx.positions, ctx.token_row, cache.block_table,
                               self.n_q_heads, self.n_kv_heads, self.head_dim, cache.page_size,

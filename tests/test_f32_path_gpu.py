@@ -1,7 +1,9 @@
-"""The products of the true 32-bit path at the edges of their kernels' ranges, against 64 bits; a row's result is the same
-bits in whatever company it comes."""
+"""The products and the attention of the true 32-bit path at the edges of their kernels' ranges, against 64 bits; a row's
+and a token's result is the same bits in whatever company it comes."""
 import pytest
 import torch
+
+from tests.test_kernels_gpu import attention_case, flat_meta
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +31,48 @@ def test_gemm_f32_rows(n, k, full):
         assert bool(((out.double() - exact[:m]).abs() <= bound[:m]).all()), m
         whole = out if whole is None else whole
         assert torch.equal(out, whole[:m]), m
+
+
+CASES = [
+    # n_q, n_kv, d, lengths, chunk starts, page, window
+    (4, 2, 128, [1, 255, 256, 257, 512, 513, 700], [0, 254, 0, 200, 511, 300, 699], 16, 0),
+    (6, 2, 32, [65, 3, 511, 1], [64, 0, 300, 0], 3, 0),
+    (3, 3, 64, [64, 65, 1025], [63, 0, 1000], 8, 0),
+    (8, 1, 64, [300, 129, 700], [250, 128, 699], 16, 100),
+    (16, 1, 128, [600, 70], [500, 69], 32, 0),
+    (64, 1, 32, [270], [200], 16, 300),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=[f"case{i}" for i in range(len(CASES))])
+def test_attention_f32(case):
+    from qwen_inference_lab_b200.kernels import attention_f32, ops
+    n_q, n_kv, d, lengths, starts, page, window = case
+    q, pool, table, meta, expected = attention_case(n_q, n_kv, d, lengths, starts, torch.float32, page, seed=5, window=window)
+    q, pool, table = q.cuda(), pool.cuda(), table.cuda()
+    as_int = lambda values: torch.tensor(values, dtype=torch.int32).cuda()
+    shape = (table, n_q, n_kv, d, page, window, d ** -0.5)
+    tile_info, single_info, at = [], [], 0
+    for start, length, pos0, row in zip(meta["seg_start"], meta["seg_len"], meta["seg_pos0"], meta["seg_row"]):
+        for off in range(0, length, 64):
+            tile_info += [start + off, pos0 + off, min(64, length - off), row]
+        single_info += [v for j in range(length) for v in (start + j, pos0 + j, row, 0)]
+    tiled, alone = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    attention_f32.tiles(q, pool, tiled, as_int(tile_info), len(tile_info) // 4, *shape)
+    n = len(single_info) // 4
+    if n_q // n_kv <= attention_f32.MOST_SINGLE_GROUP:
+        n_spans = (max(lengths) + 255) // 256 + 1                  # one spare span
+        scratch = (torch.full((n * n_q * n_spans * d,), float("nan"), device="cuda"),
+                   torch.full((n * n_q * n_spans * 2,), float("nan"), device="cuda"),
+                   torch.zeros(n * n_kv, dtype=torch.int32, device="cuda"))
+        attention_f32.singles(q, pool, alone, as_int(single_info), n, n_spans, scratch, *shape)
+        assert int(scratch[2].abs().max()) == 0
+        assert torch.equal(alone, tiled)
+    walked = torch.full_like(q, float("nan"))
+    attention_f32.tiles(q, pool, walked, as_int(single_info), n, *shape, singles=True)
+    assert torch.equal(walked, tiled)
+    torch.testing.assert_close(tiled.cpu(), expected.float(), atol=2e-6, rtol=2e-5)
+    generic = torch.empty_like(q)
+    positions, token_row = flat_meta(meta)
+    ops.attention_generic(q, pool, generic, positions, token_row, table, n_q, n_kv, d, page, window, d ** -0.5)
+    torch.testing.assert_close(tiled, generic, atol=2e-6, rtol=2e-5)
