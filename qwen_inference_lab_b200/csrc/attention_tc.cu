@@ -1,4 +1,4 @@
-// Causal grouped-query attention of whole 128-token query tiles over the paged cache on the
+// Causal grouped-query attention of query tiles of up to 128 tokens over the paged cache on the
 // fifth-generation tensor cores (tcgen05.mma, accumulators in tensor memory, operands brought by
 // TMA), for bfloat16 and one pair of sizes: -DQIL_HEAD_DIM=<of queries and keys> -DQIL_V_DIM=<of values>, each a multiple
 // of 16 up to 128 (the default of both).  Same arithmetic as attention_mma.cu (scores = q k^T *
@@ -218,10 +218,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // heads vary fastest, so all heads of the longest tile start first (tiles come sorted, longest first)
     const int head = blockIdx.x;
     const int kv_head = head / (p.n_q_heads / p.n_kv_heads);
-    // tile_info: (first token in the flat batch, its absolute position, 128, block-table row)
+    // tile_info: (first token in the flat batch, its absolute position, tokens, block-table row).  Rows past the tile's
+    // tokens hold other tokens' queries or zeros; they see what its last token sees and are not stored.
     const int4 info = tile_info[blockIdx.y];
-    const int n0 = info.x, pos0 = info.y;
-    const int hi = pos0 + AT_M - 1;                          // last key any row of the tile may see
+    const int n0 = info.x, pos0 = info.y, rows = min(info.z, AT_M);
+    const int hi = pos0 + rows - 1;                          // last key any row of the tile may see
     // the first key that the query at a position sees
     auto first_key_of = [&p](int position) {
         const int of_chunk = p.chunk > 0 ? position / p.chunk * p.chunk : 0;
@@ -372,7 +373,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     } else if (warp < AT_VALUE_WARP) {
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                 // query row of this thread = its TMEM lane
-        const int pos = pos0 + row;
+        const int pos = min(pos0 + row, hi);
         const int lo = first_key_of(pos);                     // the first key this row sees
         const unsigned lane_base = (unsigned)(quarter * 32) << 16;
         // With a distance bias the scores are scaled and biased first and the steps below take them as they are.
@@ -526,7 +527,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     bf16* o = reinterpret_cast<bf16*>(&packed);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) o[i] = __float2bfloat16_rn(__uint_as_float(r[q * 8 + i]) * inv);
-                    *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = packed;
+                    if (row < rows) *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = packed;
                 }
             }
         }
@@ -561,7 +562,7 @@ extern "C" int qil_attn_tc_keys_per_tile() { return AT_N; }
 
 // q [N, Hq, AT_D], out [N, Hq, AT_E], kv one layer's pages: a page's key rows [Hkv, page_size, AT_D] and behind them its value
 // rows [Hkv, page_size, AT_E]; all bfloat16.
-// tile_info int32 [n_tiles, 4] = (first token, its absolute position, 128, block-table row): whole tiles only.
+// tile_info int32 [n_tiles, 4] = (first token, its absolute position, tokens from 1 to 128, block-table row).
 // page_size must divide the keys per tile and be a multiple of 8.  error_word: a device int, zeroed by the
 // caller once.  trace: null, or 3 * 1024 int64 for the time stamps of block (0, 0) in a build with AT_TRACE.
 // slopes_log2: null, or float32 [n_q_heads] on the device: a distance bias per query head (see AtParams).

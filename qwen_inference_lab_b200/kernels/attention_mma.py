@@ -23,6 +23,19 @@ QUERY_TILE = 64          # tokens per query tile of ``attn_prefill_kernel``
 BIG_QUERY_TILE = attention_tc.TILE     # tokens per query tile of the tensor-memory kernel
 
 
+#: A tail's context from which on the tensor-memory kernel takes it whatever its length.  It walks a context at 1 us per
+#: 64 keys, the 64-token kernel at 2.2, and has a launch less when nothing is left to the other one; what it wastes is
+#: rows of a tile.  Measured on 32 heads of 128: a tail of 125 tokens behind 1920, 70 us of a kernel of its own against
+#: none beside three whole tiles.
+TAIL_CONTEXT = 256
+
+
+def tail_in_tile(tail, context) -> bool:
+    """Do the last ``tail`` (< 128) tokens of a segment that ends at position ``context`` - 1 make a tile of the
+    tensor-memory kernel?  More than 64 would be two tiles of the other one."""
+    return tail > QUERY_TILE or context > TAIL_CONTEXT
+
+
 PLAN_KEY = "paged_attention"     # the step planner whose arrays ``attend`` reads (``describe_segments`` makes them)
 
 
@@ -34,21 +47,25 @@ def describe_segments(first, starts, lens, rows) -> dict:
     ``tile_info``       query tiles of 64 tokens of every segment longer than one token; four ints a
                         tile: (first token in the flat batch, its absolute position, tokens in the tile,
                         block-table row)
-    ``big_tile_info``   the same segments' whole tiles of 128 tokens (for the tensor-memory kernel) ...
+    ``big_tile_info``   the same segments' tiles of 128 tokens (for the tensor-memory kernel): the whole ones, and a
+                        last one of fewer tokens where ``tail_in_tile`` says so ...
     ``rest_tile_info``  ... and 64-token tiles of what those leave over (short segments, tails)
     ``decode_info``     segments of exactly one token: (token, its position, block-table row, the longest
                         context among these segments)
 
     Tiles are sorted with the longest contexts first: they take longest, the short ones fill the gaps.
     """
-    def tiles(indices, tile, begin_of=lambda length: 0, end_of=lambda length: length):
-        found = [(first[i] + off, starts[i] + off, min(tile, end_of(int(lens[i])) - off), rows[i])
-                 for i in indices for off in range(begin_of(int(lens[i])), end_of(int(lens[i])), tile)]
+    def tiles(indices, tile, begin_of=lambda i: 0, end_of=lambda i: int(lens[i])):
+        found = [(first[i] + off, starts[i] + off, min(tile, end_of(i) - off), rows[i])
+                 for i in indices for off in range(begin_of(i), end_of(i), tile)]
         found.sort(key=lambda t: -(t[1] + t[2]))
         return np.array(found, dtype=np.int64).reshape(-1)
 
     multi = np.nonzero(lens > 1)[0]
-    whole = lambda length: length // BIG_QUERY_TILE * BIG_QUERY_TILE
+    def whole(i):
+        length = int(lens[i])
+        tail = length % BIG_QUERY_TILE
+        return length if tail and tail_in_tile(tail, int(starts[i]) + length) else length - tail
     single = np.nonzero(lens == 1)[0]
     if len(single):
         decode_info = np.stack([first[single], starts[single], rows[single],

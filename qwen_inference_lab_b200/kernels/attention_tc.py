@@ -56,7 +56,7 @@ def prefill(q, pages, out, tile_info, n_tiles, block_table, n_q_heads, n_kv_head
             lib=None, slopes_log2=None, chunk=0, sink_log2=None, softcap=0.0, window=0, head_dim=MOST_DIM, v_dim=None):
     """q bfloat16 [N, Hq*head_dim], out [N, Hq*v_dim] (``v_dim`` None: head_dim); pages [num_pages, 2, Hkv, page_size, head_dim],
     or with a value size of its own [num_pages, Hkv * page_size * (head_dim + v_dim)];
-    tile_info int32 [n_tiles * 4] = (first token, its position, 128, block-table row).
+    tile_info int32 [n_tiles * 4] = (first token, its position, tokens from 1 to 128, block-table row).
     ``slopes_log2`` float32 [Hq] on the device: slope_h * log2(e) of a bias slope_h * (query position - key
     position) taken off the scaled score.  ``chunk`` > 0: a query sees the keys of its own chunk of that many
     positions only.  ``sink_log2`` float32 [Hq] on the device: learned scores times log2(e) whose exponentials join
