@@ -74,11 +74,16 @@ __device__ __forceinline__ float2 join(float& m_run, float& l_run, float m, floa
 }
 
 // ---------------------------------------------------------------- single tokens
-// A block takes one span of one (token, kv head) and all its query heads, so that keys and values are read once; they
-// come through a ring of SINGLE_SLOTS stages of 32 rows, first the span's keys, then its values.  Spans of a token are
-// joined by the block that draws its last ticket.
+// A block takes one span of one (token, kv head) and all its query heads, so that keys and values are read once.  They
+// come through a ring of SINGLE_SLOTS stages of 16 KB: first the keys, 32 elements of 128 of them a stage (a key a
+// thread, whose sums stay in registers over the stages of a head), then the values, 4096 / D whole rows a stage (a value
+// element a thread).  Spans of a token are joined by the block that draws its last ticket.  A span that does not hold the
+// token itself asks for its first stages before the kernel before this one, which writes the token's own key and value,
+// has ended.  Bound by memory and a block's chain of stages: 8 tokens of 16 heads at contexts up to 2000 read 85 MB a
+// layer.  (Keys by whole rows, 32 of them a stage and a warp a query head, left two of four warps idle with two heads a
+// kv head: 34 us a layer; the step with this form and the chained launches around it 2.80 -> 2.35 ms.)
 #define SINGLE_THREADS 128
-#define SINGLE_ROWS 32
+#define SINGLE_STAGE 4096       // floats
 #define SINGLE_SLOTS 4
 
 template <int D, int G>     // G: query heads per kv head, rounded up
@@ -86,99 +91,126 @@ __global__ void __launch_bounds__(SINGLE_THREADS)
 attention_f32_single_kernel(const float* __restrict__ q, const Pages pages, float* __restrict__ out,
                             const int* __restrict__ info, float* part_o, float* part_ml, int* tickets,
                             int n_q_heads, int window, float scale) {
-    constexpr int LD = D + 4, PARTS = SINGLE_THREADS / D, PER = (G + PARTS - 1) / PARTS;
+    constexpr int PARTS = SINGLE_THREADS / D, PER = (G + PARTS - 1) / PARTS, CHUNKS = D / 32, VALUES = SINGLE_STAGE / D;
     extern __shared__ __align__(16) float smem[];
     long long* offsets = reinterpret_cast<long long*>(smem);               // [SPAN]
-    float* ring = smem + 2 * SPAN;                                         // [SLOTS][32][LD]
-    float* qs = ring + SINGLE_SLOTS * SINGLE_ROWS * LD;                    // [G][D]
+    float* ring = smem + 2 * SPAN;                                         // [SLOTS][STAGE]
+    float* qs = ring + SINGLE_SLOTS * SINGLE_STAGE;                        // [G][D]
     float* ps = qs + G * D;                                                // [G][SPAN]
     float* ml = ps + G * SPAN;                                             // [G][2]
     __shared__ int drawn;
-    qil_wait_for_producer();
-    qil_release_consumer();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i = blockIdx.x / pages.n_kv_heads, kv_head = blockIdx.x % pages.n_kv_heads, span = blockIdx.y;
     const int group = n_q_heads / pages.n_kv_heads;
     const int token = info[4 * i], pos = info[4 * i + 1];
     const int lo = window > 0 && pos - window + 1 > 0 ? pos - window + 1 : 0;
     const int first_span = lo / SPAN, n_spans = pos / SPAN - first_span + 1;
-    if (span < first_span || span >= first_span + n_spans) return;
+    if (span < first_span || span >= first_span + n_spans) { qil_wait_for_producer(); return; }
     const int* table = pages.block_table + (size_t)info[4 * i + 2] * pages.table_stride;
-    const int key0 = span * SPAN, begin = max(lo - key0, 0) / SINGLE_ROWS, end = min(pos - key0, SPAN - 1) / SINGLE_ROWS + 1;
-    for (int k = tid; k < SPAN; k += SINGLE_THREADS) {
-        const int key = key0 + k;
-        offsets[k] = key >= lo && key <= pos ? row_offset<D>(pages, table, kv_head, key) : -1;
-    }
-    const float* q_rows = q + ((size_t)token * n_q_heads + kv_head * group) * D;
-    for (int k = tid; k < G * D; k += SINGLE_THREADS) qs[k] = k < group * D ? q_rows[k] : 0.f;
+    const int key0 = span * SPAN, from_key = max(lo - key0, 0), last_key = min(pos - key0, SPAN - 1);
+    for (int k = tid; k < SPAN; k += SINGLE_THREADS)
+        offsets[k] = k >= from_key && k <= last_key ? row_offset<D>(pages, table, kv_head, key0 + k) : -1;
     for (int k = tid; k < G * SPAN; k += SINGLE_THREADS) ps[k] = -INFINITY;
     __syncthreads();
 
-    const int n_sub = end - begin;
+    const int k_begin = from_key / SINGLE_THREADS, k_stages = (last_key / SINGLE_THREADS + 1 - k_begin) * CHUNKS;
+    const int v_begin = from_key / VALUES, n_stages = k_stages + last_key / VALUES + 1 - v_begin;
     const long long plane = (long long)pages.n_kv_heads * pages.page_size * D;
-    auto load = [&](int stage) {       // stages 0 .. n_sub - 1 are the keys, the rest the values
-        if (stage < 2 * n_sub) {
-            float* to = ring + stage % SINGLE_SLOTS * SINGLE_ROWS * LD;
-            const int rows0 = (begin + (stage < n_sub ? stage : stage - n_sub)) * SINGLE_ROWS;
-            const float* from = pages.cache + (stage < n_sub ? 0 : plane);
+    auto load = [&](int stage) {
+        if (stage < n_stages) {
+            float* to = ring + stage % SINGLE_SLOTS * SINGLE_STAGE;
+            if (stage < k_stages) {
+                // a key's 8 pieces of 16 bytes lie in an order of its own: 8 threads that read one piece of 8 keys each
+                // then meet every bank once
+                const int row0 = (k_begin + stage / CHUNKS) * SINGLE_THREADS;
+                const float* from = pages.cache + stage % CHUNKS * 32;
 #pragma unroll
-            for (int idx = tid; idx < SINGLE_ROWS * (D / 4); idx += SINGLE_THREADS) {
-                const int row = idx / (D / 4), col = idx % (D / 4) * 4;
-                const long long at = offsets[rows0 + row];
-                copy16(to + row * LD + col, at >= 0 ? from + at + col : pages.cache, at >= 0);
+                for (int n = 0; n < SINGLE_STAGE / 4 / SINGLE_THREADS; ++n) {
+                    const int row = n * 16 + (tid >> 3), piece = tid & 7;
+                    const long long at = offsets[row0 + row];
+                    copy16(to + row * 32 + (piece ^ (row & 7)) * 4, at >= 0 ? from + at + piece * 4 : pages.cache, at >= 0);
+                }
+            } else {
+                const int row0 = (v_begin + stage - k_stages) * VALUES;
+#pragma unroll
+                for (int n = 0; n < SINGLE_STAGE / 4 / SINGLE_THREADS; ++n) {
+                    const int idx = n * SINGLE_THREADS + tid, row = idx / (D / 4), col = idx % (D / 4) * 4;
+                    const long long at = offsets[row0 + row];
+                    copy16(to + row * D + col, at >= 0 ? pages.cache + plane + at + col : pages.cache, at >= 0);
+                }
             }
         }
         copies_commit();
     };
-    for (int s = 0; s < SINGLE_SLOTS - 1; ++s) load(s);
+    const bool early = pos - key0 >= SPAN;
+    if (early)
+        for (int s = 0; s < SINGLE_SLOTS - 1; ++s) load(s);
+    qil_wait_for_producer();
+    qil_release_consumer();
+    if (!early)
+        for (int s = 0; s < SINGLE_SLOTS - 1; ++s) load(s);
+    const float* q_rows = q + ((size_t)token * n_q_heads + kv_head * group) * D;
+    for (int k = tid; k < G * D; k += SINGLE_THREADS) qs[k] = k < group * D ? q_rows[k] : 0.f;
 
+    unsigned long long dot[G];
+#pragma unroll
+    for (int r = 0; r < G; ++r) dot[r] = 0ull;
+    for (int s = 0; s < k_stages; ++s) {
+        copies_wait<SINGLE_SLOTS - 2>();
+        __syncthreads();
+        load(s + SINGLE_SLOTS - 1);
+        const float* row = ring + s % SINGLE_SLOTS * SINGLE_STAGE + tid * 32;
+        const float* qc = qs + s % CHUNKS * 32;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(row + (c ^ (tid & 7)) * 4);
+#pragma unroll
+            for (int r = 0; r < G; ++r) {
+                const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qc + r * D + c * 4);
+                fma_pair(dot[r], q4.x, k4.x);
+                fma_pair(dot[r], q4.y, k4.y);
+            }
+        }
+        if (s % CHUNKS == CHUNKS - 1) {
+            const int k = (k_begin + s / CHUNKS) * SINGLE_THREADS + tid;
+            const bool there = offsets[k] >= 0;
+#pragma unroll
+            for (int r = 0; r < G; ++r) {
+                const float2 halves = pair_of(dot[r]);
+                if (there) ps[r * SPAN + k] = (halves.x + halves.y) * scale;
+                dot[r] = 0ull;
+            }
+        }
+    }
+    __syncthreads();
+    for (int r = warp; r < group; r += SINGLE_THREADS / 32) {
+        const float2 v = span_softmax(ps + r * SPAN, lane);
+        if (lane == 0) { ml[2 * r] = v.x; ml[2 * r + 1] = v.y; }
+    }
     float acc[PER];
 #pragma unroll
     for (int r = 0; r < PER; ++r) acc[r] = 0.f;
     const int d = tid % D, part = tid / D;      // a thread sums one value element of every PARTS-th query head
-    for (int s = 0; s < 2 * n_sub; ++s) {
+    for (int s = k_stages; s < n_stages; ++s) {
         copies_wait<SINGLE_SLOTS - 2>();
-        if (s == n_sub) {                       // all scores are there
-            __syncthreads();
-            for (int r = warp; r < group; r += SINGLE_THREADS / 32) {
-                const float2 v = span_softmax(ps + r * SPAN, lane);
-                if (lane == 0) { ml[2 * r] = v.x; ml[2 * r + 1] = v.y; }
-            }
-        }
         __syncthreads();
         load(s + SINGLE_SLOTS - 1);
-        const float* rows = ring + s % SINGLE_SLOTS * SINGLE_ROWS * LD;
-        const int k0 = (begin + (s < n_sub ? s : s - n_sub)) * SINGLE_ROWS;
-        if (s < n_sub) {
-            // a key a lane; the warps share the query heads out
-            const float* row = rows + lane * LD;
-            for (int r = warp; r < group; r += SINGLE_THREADS / 32) {
-                unsigned long long dot = 0ull;
-#pragma unroll 8
-                for (int c = 0; c < D; c += 4) {
-                    const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(row + c);
-                    const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qs + r * D + c);
-                    fma_pair(dot, q4.x, k4.x);
-                    fma_pair(dot, q4.y, k4.y);
-                }
-                const float2 halves = pair_of(dot);
-                if (offsets[k0 + lane] >= 0) ps[r * SPAN + k0 + lane] = (halves.x + halves.y) * scale;
-            }
-        } else {
-            const int last = min(SINGLE_ROWS, pos - key0 - k0 + 1);
-            for (int k = 0; k < last; k += 4) {      // rows past the last key are zeros with weight zero
-                float v[4];
+        const float* rows = ring + s % SINGLE_SLOTS * SINGLE_STAGE + d;
+        const int k0 = (v_begin + s - k_stages) * VALUES;
+        const int last = min(VALUES, last_key - k0 + 1);
+#pragma unroll 4
+        for (int k = 0; k < last; k += 4) {     // rows past the last key are zeros with weight zero
+            float v[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = rows[(k + e) * LD + d];
+            for (int e = 0; e < 4; ++e) v[e] = rows[(k + e) * D];
 #pragma unroll
-                for (int r = 0; r < PER; ++r) {
-                    if (part + r * PARTS >= G) continue;
-                    const float4 p = *reinterpret_cast<const float4*>(ps + (part + r * PARTS) * SPAN + k0 + k);
-                    acc[r] = fmaf(p.x, v[0], acc[r]);
-                    acc[r] = fmaf(p.y, v[1], acc[r]);
-                    acc[r] = fmaf(p.z, v[2], acc[r]);
-                    acc[r] = fmaf(p.w, v[3], acc[r]);
-                }
+            for (int r = 0; r < PER; ++r) {
+                if (part + r * PARTS >= G) continue;
+                const float4 p = *reinterpret_cast<const float4*>(ps + (part + r * PARTS) * SPAN + k0 + k);
+                acc[r] = fmaf(p.x, v[0], acc[r]);
+                acc[r] = fmaf(p.y, v[1], acc[r]);
+                acc[r] = fmaf(p.z, v[2], acc[r]);
+                acc[r] = fmaf(p.w, v[3], acc[r]);
             }
         }
     }
@@ -421,7 +453,7 @@ static int launch(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream
 template <int D, int G>
 static int launch_single(const float* q, const Pages& pages, float* out, const int* info, int n, int n_spans, float* part_o,
                          float* part_ml, int* tickets, int n_q_heads, int window, float scale, cudaStream_t stream) {
-    const size_t smem = (size_t)(2 * SPAN + SINGLE_SLOTS * SINGLE_ROWS * (D + 4) + G * (D + SPAN + 2)) * sizeof(float);
+    const size_t smem = (size_t)(2 * SPAN + SINGLE_SLOTS * SINGLE_STAGE + G * (D + SPAN + 2)) * sizeof(float);
     return launch(attention_f32_single_kernel<D, G>, dim3(n * pages.n_kv_heads, n_spans), SINGLE_THREADS, smem, stream, q, pages,
                   out, info, part_o, part_ml, tickets, n_q_heads, window, scale);
 }

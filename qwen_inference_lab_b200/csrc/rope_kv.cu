@@ -22,6 +22,8 @@ __global__ void qk_norm_rope_store_kernel(
     const int* __restrict__ block_table, int table_stride,
     int n_q_heads, int n_kv_heads, int head_dim, int page_size, int num_pages) {
     extern __shared__ float stage[];  // [warps][head_dim]
+    qil_wait_for_producer();
+    qil_release_consumer();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int token = blockIdx.x;
     const int head = blockIdx.y * (blockDim.x >> 5) + warp;
@@ -260,7 +262,7 @@ extern "C" int qil_qk_norm_rope_store(
     dim3 grid(n_tokens, (total_heads + warps - 1) / warps);
     const size_t smem = (size_t)warps * head_dim * sizeof(float);
     QIL_DISPATCH_2(act_dtype, norm_w_dtype,
-        (qk_norm_rope_store_kernel<T, W><<<grid, warps * 32, smem, stream>>>(
+        (qil_launch_chained(qk_norm_rope_store_kernel<T, W>, grid, dim3(warps * 32), smem, stream,
             (const T*)qkv, (T*)q_out, (T*)kv_cache, (const W*)q_norm_w, (const W*)k_norm_w, eps,
             rope_table, rotary_dim, table_rows, positions, token_row, block_table, table_stride,
             n_q_heads, n_kv_heads, head_dim, page_size, num_pages)));
