@@ -151,8 +151,8 @@ rmsnorm_bf16x8_kernel(const bf16* __restrict__ x, const W* __restrict__ weight, 
 }
 
 // float32 rows of up to 256 * RMS_F32_VPT elements: the same sums and products as rmsnorm_kernel (thread t takes elements
-// t, t + 256, ...), with all of a row's loads in flight at once and the row read once.  A decode step's rows cost a
-// launch and a trip to memory and no more: 8 rows of 1024 3.9 us in a chain of ordinary launches, 2.4 chained.
+// t, t + 256, ...), with all of a row's loads in flight at once and the row read once: what a decode step's rows cost is
+// a launch and a trip to memory.
 #define RMS_F32_VPT 16
 __global__ void __launch_bounds__(256)
 rmsnorm_f32_kernel(const float* __restrict__ x, const float* __restrict__ weight, const int* __restrict__ rows,
