@@ -182,18 +182,20 @@ gemm_f32_stream_kernel(const GemmArgs g, int stages) {
     cluster_barrier();      // no block leaves while another reads its sums
 }
 
-// More rows: 8 x 4 outputs a thread, tiles of BM x 64, both operands through a ring of stages of 16 k as they lie in
+// More rows: 8 x 4 outputs a thread, tiles of BM x 64, both operands through a ring of stages of 32 k as they lie in
 // memory (k innermost, so that a 16-byte read is two packed FMA operands and nothing is transposed or duplicated).
 // Without a cluster a block adds its runs' sums up in shared memory; a cluster of GEMM_RUNS takes one run a block.
-// Bound by the FMA pipe's issue: 27 TFLOP/s at 512 rows whether a thread holds 8 x 8 or 8 x 4 outputs (6.4 or 12 warps
-// an SM); 8 x 4 leaves three blocks an SM and finer tiles for few rows.  Unpipelined 64 x 64 x 16 tiles with scalar FMA: 9.
+// Bound by the 16-byte reads of shared memory, each of which returns 512 bytes to a warp whether its lanes share them or
+// not: scalar FMA, packed FMA and 8 x 8 outputs a thread all end within 5 %.  So the reads run ahead of the FMA by four k
+// and a stage holds 32 k (a barrier half as often): 512 x 6144 x 1024 237 -> 196 us (33 TFLOP/s), 512 x 1024 x 3072 124 ->
+// 100; unpipelined 64 x 64 x 16 tiles with scalar FMA ran at 9 TFLOP/s.
 #define TILE_BN 64
-#define TILE_BK 16
+#define TILE_BK 32
 #define TILE_LD (TILE_BK + 4)
-#define TILE_STAGES 3
+#define TILE_STAGES 2
 
 template <int BM>
-__global__ void __launch_bounds__(BM * 2)
+__global__ void __launch_bounds__(BM * 2, BM == 64 ? 3 : 6)
 gemm_f32_tile_kernel(const GemmArgs g) {
     constexpr int J = TILE_BN / 16, THREADS = BM * 2, TY = BM / 8, STAGE = (BM + TILE_BN) * TILE_LD;
     extern __shared__ __align__(16) float smem[];
@@ -217,8 +219,8 @@ gemm_f32_tile_kernel(const GemmArgs g) {
             float* to = smem + stage % TILE_STAGES * STAGE;
             const int k0 = k_begin + stage * TILE_BK;
 #pragma unroll
-            for (int i = 0; i < (BM + TILE_BN) * 4 / THREADS; ++i) {
-                const int idx = tid + i * THREADS, row = idx >> 2, k = k0 + (idx & 3) * 4;
+            for (int i = 0; i < (BM + TILE_BN) * 8 / THREADS; ++i) {
+                const int idx = tid + i * THREADS, row = idx >> 3, k = k0 + (idx & 7) * 4;
                 const float* from;
                 bool inside = k < k_end;
                 if (row < BM) {
@@ -228,7 +230,7 @@ gemm_f32_tile_kernel(const GemmArgs g) {
                     inside = inside && n0 + row - BM < g.N;
                     from = g.W + (size_t)(n0 + row - BM) * g.K + k;
                 }
-                copy16(to + row * TILE_LD + (idx & 3) * 4, inside ? from : g.W, inside);
+                copy16(to + row * TILE_LD + (idx & 7) * 4, inside ? from : g.W, inside);
             }
         }
         copies_commit();
@@ -246,19 +248,26 @@ gemm_f32_tile_kernel(const GemmArgs g) {
         load(s + TILE_STAGES - 1);
         const float* as = smem + s % TILE_STAGES * STAGE + ty * TILE_LD;
         const float* ws = smem + s % TILE_STAGES * STAGE + (BM + tx) * TILE_LD;
-#pragma unroll 2
+        // the next four k's operands are read while these four multiply
+        ulonglong2 w[2][J], a[2][8];
+        auto read = [&](int q) {
+#pragma unroll
+            for (int j = 0; j < J; ++j) w[q & 1][j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * TILE_LD + q * 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[q & 1][i] = *reinterpret_cast<const ulonglong2*>(as + i * TY * TILE_LD + q * 4);
+        };
+        read(0);
+#pragma unroll
         for (int q = 0; q < TILE_BK / 4; ++q) {
-            ulonglong2 w[J];
+            if (q + 1 < TILE_BK / 4) read(q + 1);
 #pragma unroll
-            for (int j = 0; j < J; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * TILE_LD + q * 4);
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + i * TY * TILE_LD + q * 4);
+                for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a[q & 1][i].x, w[q & 1][j].x);
 #pragma unroll
-                for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a.x, w[j].x);
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a.y, w[j].y);
-            }
+                for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a[q & 1][i].y, w[q & 1][j].y);
         }
         if (blocks == 1 && ((s + 1) % run_stages == 0 || s + 1 == n_stages)) {
             const bool first = s < run_stages, last = s + 1 == n_stages;
