@@ -258,11 +258,13 @@ attention_f32_single_kernel(const float* __restrict__ q, const Pages pages, floa
 }
 
 // ---------------------------------------------------------------- prompt portions
-// A block takes 64 query rows (the query heads of a kv head for as many consecutive tokens) and walks the spans.  Scores
-// of a span sit in shared memory: 4 x 4 of them a thread and 64-key stage; then 4 value elements of 64 * D / 1024 rows a
-// thread.  Stages of 64 rows come through a ring of TILE_SLOTS.
+// A block takes 64 query rows (the query heads of a kv head for as many consecutive tokens) and walks the spans.  A span's
+// keys come 32 elements at a time, all 256 of them a stage of 32 KB, and a thread holds 8 x 8 scores over the stages of a
+// head; its values come 8192 / D rows a stage, and a thread holds 4 elements of 64 * D / 1024 rows.  Bound by the 16-byte
+// reads of shared memory, each of which returns 512 bytes to a warp whether its lanes share them or not.
 #define TILE_THREADS 256
 #define TILE_ROWS 64
+#define TILE_STAGE 8192         // floats
 #define TILE_SLOTS 3
 #define SCORE_LD (SPAN + 4)
 
@@ -270,11 +272,11 @@ template <int D>
 __global__ void __launch_bounds__(TILE_THREADS)
 attention_f32_tile_kernel(const float* __restrict__ q, const Pages pages, float* __restrict__ out,
                           const int* __restrict__ info, int n_subtiles, int singles, int n_q_heads, int window, float scale) {
-    constexpr int LD = D + 4, GROUPS = TILE_THREADS / (D / 4), PER = TILE_ROWS / GROUPS;
+    constexpr int LD = D + 4, GROUPS = TILE_THREADS / (D / 4), PER = TILE_ROWS / GROUPS, CHUNKS = D / 32, VALUES = TILE_STAGE / D;
     extern __shared__ __align__(16) float smem[];
     long long* offsets = reinterpret_cast<long long*>(smem);               // [SPAN]
-    float* ring = smem + 2 * SPAN;                                         // [SLOTS][64][LD]
-    float* qs = ring + TILE_SLOTS * TILE_ROWS * LD;                        // [64][LD]
+    float* ring = smem + 2 * SPAN;                                         // [SLOTS][STAGE]
+    float* qs = ring + TILE_SLOTS * TILE_STAGE;                            // [64][LD]
     float* ps = qs + TILE_ROWS * LD;                                       // [64][SCORE_LD]
     float* ml = ps + TILE_ROWS * SCORE_LD;                                 // [64][2]
     qil_wait_for_producer();
@@ -296,9 +298,9 @@ attention_f32_tile_kernel(const float* __restrict__ q, const Pages pages, float*
             v = *reinterpret_cast<const float4*>(q + ((size_t)(token0 + row / group) * n_q_heads + kv_head * group + row % group) * D + col);
         *reinterpret_cast<float4*>(qs + row * LD + col) = v;
     }
-    // scores: rows ry + 16 i, keys kx + 16 j of a stage (a warp holds 4 x 8 threads); values: columns d .. d + 3 of
+    // scores: rows ry + 8 i, keys kx + 32 j of a span (a warp holds 4 x 8 threads); values: columns d .. d + 3 of
     // rows row0 .. row0 + PER - 1
-    const int ry = (warp >> 1) * 4 + (lane >> 3), kx = (warp & 1) * 8 + (lane & 7);
+    const int ry = (warp >> 2) * 4 + (lane >> 3), kx = (warp & 3) * 8 + (lane & 7);
     const int d = tid % (D / 4) * 4, row0 = tid / (D / 4) * PER;
     const long long plane = (long long)pages.n_kv_heads * pages.page_size * D;
     float m_run[PER], l_run[PER], o_run[PER][4];
@@ -310,106 +312,132 @@ attention_f32_tile_kernel(const float* __restrict__ q, const Pages pages, float*
     }
 
     for (int span = lo / SPAN; span <= hi / SPAN; ++span) {
-        const int key0 = span * SPAN, begin = max(lo - key0, 0) / TILE_ROWS, end = min(hi - key0, SPAN - 1) / TILE_ROWS + 1;
-        const int n_sub = end - begin;
+        const int key0 = span * SPAN, from_key = max(lo - key0, 0), last_key = min(hi - key0, SPAN - 1);
+        const int v_begin = from_key / VALUES, n_stages = CHUNKS + last_key / VALUES + 1 - v_begin;
         __syncthreads();                        // the span before is read out
-        for (int k = tid; k < SPAN; k += TILE_THREADS) {
-            const int key = key0 + k;
-            offsets[k] = key >= lo && key <= hi ? row_offset<D>(pages, table, kv_head, key) : -1;
-        }
+        for (int k = tid; k < SPAN; k += TILE_THREADS)
+            offsets[k] = k >= from_key && k <= last_key ? row_offset<D>(pages, table, kv_head, key0 + k) : -1;
         for (int idx = tid; idx < TILE_ROWS * (SCORE_LD / 4); idx += TILE_THREADS)
             reinterpret_cast<float4*>(ps)[idx] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
         __syncthreads();
-        auto load = [&](int stage) {            // stages 0 .. n_sub - 1 are the keys, the rest the values
-            if (stage < 2 * n_sub) {
-                float* to = ring + stage % TILE_SLOTS * TILE_ROWS * LD;
-                const int rows0 = (begin + (stage < n_sub ? stage : stage - n_sub)) * TILE_ROWS;
-                const float* from = pages.cache + (stage < n_sub ? 0 : plane);
-#pragma unroll 4
-                for (int idx = tid; idx < TILE_ROWS * (D / 4); idx += TILE_THREADS) {
-                    const int row = idx / (D / 4), col = idx % (D / 4) * 4;
-                    const long long at = offsets[rows0 + row];
-                    copy16(to + row * LD + col, at >= 0 ? from + at + col : pages.cache, at >= 0);
+        auto load = [&](int stage) {            // the first CHUNKS stages are the keys, the rest the values
+            if (stage < n_stages) {
+                float* to = ring + stage % TILE_SLOTS * TILE_STAGE;
+                if (stage < CHUNKS) {
+                    // a key's 8 pieces of 16 bytes lie in an order of its own, as in the kernel above
+#pragma unroll
+                    for (int n = 0; n < SPAN * 8 / TILE_THREADS; ++n) {
+                        const int row = n * (TILE_THREADS / 8) + (tid >> 3), piece = tid & 7;
+                        const long long at = offsets[row];
+                        copy16(to + row * 32 + (piece ^ (row & 7)) * 4, at >= 0 ? pages.cache + at + stage * 32 + piece * 4 : pages.cache, at >= 0);
+                    }
+                } else {
+                    const int rows0 = (v_begin + stage - CHUNKS) * VALUES;
+#pragma unroll
+                    for (int n = 0; n < TILE_STAGE / 4 / TILE_THREADS; ++n) {
+                        const int idx = n * TILE_THREADS + tid, row = idx / (D / 4), col = idx % (D / 4) * 4;
+                        const long long at = offsets[rows0 + row];
+                        copy16(to + row * D + col, at >= 0 ? pages.cache + plane + at + col : pages.cache, at >= 0);
+                    }
                 }
             }
             copies_commit();
         };
         for (int s = 0; s < TILE_SLOTS - 1; ++s) load(s);
+        {
+            const int j_begin = from_key / 32, j_end = last_key / 32 + 1;       // 32 keys that hold none are left out
+            unsigned long long dot[8][8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dot[i][j] = 0ull;
+            for (int s = 0; s < CHUNKS; ++s) {
+                copies_wait<TILE_SLOTS - 2>();
+                __syncthreads();
+                load(s + TILE_SLOTS - 1);
+                const float* stage = ring + s % TILE_SLOTS * TILE_STAGE + kx * 32;
+                const float* qc = qs + ry * LD + s * 32;
+#pragma unroll 2
+                for (int c = 0; c < 8; ++c) {
+                    ulonglong2 q4[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) q4[i] = *reinterpret_cast<const ulonglong2*>(qc + i * 8 * LD + c * 4);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (j < j_begin || j >= j_end) continue;
+                        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(stage + j * 32 * 32 + (c ^ (kx & 7)) * 4);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) fma_pair(dot[i][j], q4[i].x, k4.x);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) fma_pair(dot[i][j], q4[i].y, k4.y);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int k = kx + 32 * j, key = key0 + k;
+                const bool there = offsets[k] >= 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int row = ry + 8 * i, pos = pos0 + row / group;
+                    const float2 halves = pair_of(dot[i][j]);
+                    if (there && row < rows && key <= pos && key >= low(pos)) ps[row * SCORE_LD + k] = (halves.x + halves.y) * scale;
+                }
+            }
+        }
+        __syncthreads();
+        for (int r = warp; r < rows; r += TILE_THREADS / 32) {
+            const float2 v = span_softmax(ps + r * SCORE_LD, lane);
+            if (lane == 0) { ml[2 * r] = v.x; ml[2 * r + 1] = v.y; }
+        }
         unsigned long long acc[PER][2];
 #pragma unroll
         for (int r = 0; r < PER; ++r) acc[r][0] = acc[r][1] = 0ull;
-        for (int s = 0; s < 2 * n_sub; ++s) {
+        for (int s = CHUNKS; s < n_stages; ++s) {
             copies_wait<TILE_SLOTS - 2>();
-            if (s == n_sub) {
-                __syncthreads();
-                for (int r = warp; r < rows; r += TILE_THREADS / 32) {
-                    const float2 v = span_softmax(ps + r * SCORE_LD, lane);
-                    if (lane == 0) { ml[2 * r] = v.x; ml[2 * r + 1] = v.y; }
-                }
-            }
             __syncthreads();
             load(s + TILE_SLOTS - 1);
-            const float* stage = ring + s % TILE_SLOTS * TILE_ROWS * LD;
-            const int k0 = (begin + (s < n_sub ? s : s - n_sub)) * TILE_ROWS;
-            if (s < n_sub) {
-                unsigned long long dot[4][4];
+            const float* stage = ring + s % TILE_SLOTS * TILE_STAGE + d;
+            const int k0 = (v_begin + s - CHUNKS) * VALUES;
+            // where every key of the stage is seen by every row no key is skipped; elsewhere a key that a row does not see
+            // must not reach its sum even with weight zero (its value may be an infinity)
+            if (key0 + k0 + VALUES - 1 <= pos0 && key0 + k0 >= low(hi)) {
+#pragma unroll 2
+                for (int k = 0; k < VALUES; k += 4) {
+                    ulonglong2 v[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                    for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const ulonglong2*>(stage + (k + e) * D);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) dot[i][j] = 0ull;
-#pragma unroll 4
-                for (int c = 0; c < D; c += 4) {
-                    ulonglong2 k4[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const ulonglong2*>(stage + (kx + 16 * j) * LD + c);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(qs + (ry + 16 * i) * LD + c);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) { fma_pair(dot[i][j], q4.x, k4[j].x); fma_pair(dot[i][j], q4.y, k4[j].y); }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int k = k0 + kx + 16 * j, key = key0 + k;
-                    const bool there = offsets[k] >= 0;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int row = ry + 16 * i, pos = pos0 + row / group;
-                        const float2 halves = pair_of(dot[i][j]);
-                        if (there && row < rows && key <= pos && key >= low(pos)) ps[row * SCORE_LD + k] = (halves.x + halves.y) * scale;
+                    for (int r = 0; r < PER; ++r) {
+                        const float4 p = *reinterpret_cast<const float4*>(ps + (row0 + r) * SCORE_LD + k0 + k);
+                        fma_pair(acc[r][0], twice(p.x), v[0].x); fma_pair(acc[r][1], twice(p.x), v[0].y);
+                        fma_pair(acc[r][0], twice(p.y), v[1].x); fma_pair(acc[r][1], twice(p.y), v[1].y);
+                        fma_pair(acc[r][0], twice(p.z), v[2].x); fma_pair(acc[r][1], twice(p.z), v[2].y);
+                        fma_pair(acc[r][0], twice(p.w), v[3].x); fma_pair(acc[r][1], twice(p.w), v[3].y);
                     }
                 }
             } else {
-                // where every key of the stage is seen by every row no key is skipped; elsewhere a key that a row does
-                // not see must not reach its sum even with weight zero (its value may be an infinity)
-                const bool all = key0 + k0 + TILE_ROWS - 1 <= pos0 && key0 + k0 >= low(hi);
-                if (all) {
-#pragma unroll 2
-                    for (int k = 0; k < TILE_ROWS; k += 4) {
-                        ulonglong2 v[4];
+                // four rows at a time over the keys that any of them sees
+                constexpr int Q = PER < 4 ? PER : 4;
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const ulonglong2*>(stage + (k + e) * LD + d);
+                for (int r0 = 0; r0 < PER; r0 += Q) {
+                    int from[Q], to[Q], first = VALUES, end = 0;
 #pragma unroll
-                        for (int r = 0; r < PER; ++r) {
-                            const float4 p = *reinterpret_cast<const float4*>(ps + (row0 + r) * SCORE_LD + k0 + k);
-                            fma_pair(acc[r][0], twice(p.x), v[0].x); fma_pair(acc[r][1], twice(p.x), v[0].y);
-                            fma_pair(acc[r][0], twice(p.y), v[1].x); fma_pair(acc[r][1], twice(p.y), v[1].y);
-                            fma_pair(acc[r][0], twice(p.z), v[2].x); fma_pair(acc[r][1], twice(p.z), v[2].y);
-                            fma_pair(acc[r][0], twice(p.w), v[3].x); fma_pair(acc[r][1], twice(p.w), v[3].y);
-                        }
+                    for (int r = 0; r < Q; ++r) {
+                        const int pos = pos0 + (row0 + r0 + r) / group;
+                        from[r] = max(0, low(pos) - key0 - k0);
+                        to[r] = row0 + r0 + r < rows ? min(VALUES, pos - key0 - k0 + 1) : 0;
+                        first = min(first, from[r]);
+                        end = max(end, to[r]);
                     }
-                } else {
+                    for (int k = first; k < end; ++k) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(stage + k * D);
 #pragma unroll
-                    for (int r = 0; r < PER; ++r) {
-                        if (row0 + r >= rows) continue;
-                        const int pos = pos0 + (row0 + r) / group;
-                        const int from = max(0, low(pos) - key0 - k0), to = min(TILE_ROWS, pos - key0 - k0 + 1);
-                        for (int k = from; k < to; ++k) {
-                            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(stage + k * LD + d);
-                            const unsigned long long p = twice(ps[(row0 + r) * SCORE_LD + k0 + k]);
-                            fma_pair(acc[r][0], p, v.x); fma_pair(acc[r][1], p, v.y);
-                        }
+                        for (int r = 0; r < Q; ++r)
+                            if (k >= from[r] && k < to[r]) {
+                                const unsigned long long p = twice(ps[(row0 + r0 + r) * SCORE_LD + k0 + k]);
+                                fma_pair(acc[r0 + r][0], p, v.x); fma_pair(acc[r0 + r][1], p, v.y);
+                            }
                     }
                 }
             }
@@ -461,7 +489,7 @@ static int launch_single(const float* q, const Pages& pages, float* out, const i
 template <int D>
 static int launch_tile(const float* q, const Pages& pages, float* out, const int* info, int n, int singles, int tile_tokens,
                        int n_q_heads, int window, float scale, cudaStream_t stream) {
-    const size_t smem = (size_t)(2 * SPAN + (TILE_SLOTS + 1) * TILE_ROWS * (D + 4) + TILE_ROWS * (SCORE_LD + 2)) * sizeof(float);
+    const size_t smem = (size_t)(2 * SPAN + TILE_SLOTS * TILE_STAGE + TILE_ROWS * (D + 4) + TILE_ROWS * (SCORE_LD + 2)) * sizeof(float);
     const int per_tile = TILE_ROWS / (n_q_heads / pages.n_kv_heads), subtiles = singles ? 1 : (tile_tokens + per_tile - 1) / per_tile;
     return launch(attention_f32_tile_kernel<D>, dim3(n * subtiles, pages.n_kv_heads), TILE_THREADS, smem, stream, q, pages, out, info,
                   subtiles, singles, n_q_heads, window, scale);
