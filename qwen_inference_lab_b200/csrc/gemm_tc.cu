@@ -592,6 +592,221 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
+// ------------------------------------------------------------------ a few dozen rows
+// The product for the rows between a decode step's and a prompt portion's (17 to 128): its time is that of reading W
+// once, as for the decode product, but there are too many rows for mma.sync to keep up.  128 output features sit on the
+// 128 lanes of the accumulator and the rows on its columns (W is the MMA's A operand), so a block's MMAs cost what the
+// rows need and a stage is nearly all weights.  One tile a block and nothing persistent: what counts is that every SM
+// streams from the first to the last microsecond.  So
+//   - a cluster of up to eight blocks cuts a tile's K; every block leaves its float32 sums in its shared memory and adds
+//     up, in block order, its share of the rows out of all of them (the same bits on every launch);
+//   - two blocks fit an SM, and a launch chained to the kernel before it has its barriers and tensor memory set up and its
+//     ring full of weights when that kernel ends.  (Dependents are released only when the block holds its tensor
+//     memory: blocks of a later launch never hold what blocks of an earlier one wait for.)
+// Waits are bounded as above.  Measured beside the rule that cuts K, in qil_gemm_tc_rows.
+#define TR_BM 128
+#define TR_W_BYTES (TR_BM * TC_BK * 2)
+#define TR_MOST_STAGES 6
+#define TR_MOST_BLOCKS 8
+
+struct TrShared {
+    unsigned long long full[TR_MOST_STAGES];
+    unsigned long long empty[TR_MOST_STAGES];
+    unsigned long long acc_full;
+    unsigned tmem_base;
+    unsigned pad;
+};
+
+// ROWS columns of accumulator: M <= ROWS
+template <int ROWS>
+struct TrShape {
+    static constexpr int X_BYTES = ROWS * TC_BK * 2;
+    static constexpr int STAGE_BYTES = TR_W_BYTES + X_BYTES;
+    static constexpr int STAGES = ROWS <= 32 ? 5 : ROWS <= 64 ? 4 : 3;         // two blocks an SM
+    static constexpr int SMEM = STAGES * STAGE_BYTES + (int)sizeof(TrShared) + 1024;
+};
+
+__device__ __forceinline__ float4 cluster_read4(const float* at, unsigned rank) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(map_to_rank(smem_u32(at), rank)) : "memory");
+    return v;
+}
+
+template <int ROWS, bool PAIRS>
+__global__ void __launch_bounds__(192, 2)
+gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                    const bf16* __restrict__ bias, const bf16* residual, bf16* out,
+                    int M, int N, int K, int* error_word) {
+    typedef TrShape<ROWS> Shape;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    TrShared* sh = reinterpret_cast<TrShared*>(ring + Shape::STAGES * Shape::STAGE_BYTES);
+    float* sums = reinterpret_cast<float*>(ring);          // [ROWS][128] once the ring is read out
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    unsigned blocks;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(blocks));
+    const int n0 = blockIdx.x / blocks * TR_BM;
+    const int k_blocks = (K + TC_BK - 1) / TC_BK;
+    const int kb0 = (int)((long long)k_blocks * rank / blocks), kb1 = (int)((long long)k_blocks * (rank + 1) / blocks);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < Shape::STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
+        mbar_init(&sh->acc_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                     ::"r"(smem_u32(&sh->tmem_base)), "r"((unsigned)ROWS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem_base = sh->tmem_base;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // the ring's first round: weights, which no kernel writes, before the kernel before this one has ended
+            const int first = kb1 - kb0 < Shape::STAGES ? kb1 - kb0 : Shape::STAGES;
+            for (int s = 0; s < first; ++s) {
+                mbar_arrive_expect_tx(&sh->full[s], Shape::STAGE_BYTES);
+                tma_load_2d_stream(ring + s * Shape::STAGE_BYTES, &map_w, &sh->full[s], (kb0 + s) * TC_BK, n0);
+            }
+            qil_wait_for_producer();
+            qil_release_consumer();
+            for (int s = 0; s < first; ++s)
+                tma_load_2d(ring + s * Shape::STAGE_BYTES + TR_W_BYTES, &map_x, &sh->full[s], (kb0 + s) * TC_BK, 0);
+            int stage = first == Shape::STAGES ? 0 : first;
+            unsigned phase = first == Shape::STAGES ? 1 : 0;
+            for (int kb = kb0 + first; kb < kb1; ++kb) {
+                if (!mbar_wait(&sh->empty[stage], phase ^ 1)) { atomicExch(error_word, 1); break; }
+                mbar_arrive_expect_tx(&sh->full[stage], Shape::STAGE_BYTES);
+                unsigned char* to = ring + stage * Shape::STAGE_BYTES;
+                tma_load_2d_stream(to, &map_w, &sh->full[stage], kb * TC_BK, n0);
+                tma_load_2d(to + TR_W_BYTES, &map_x, &sh->full[stage], kb * TC_BK, 0);
+                if (++stage == Shape::STAGES) { stage = 0; phase ^= 1; }
+            }
+            for (int i = 0; i < first; ++i) {      // copies in flight land before the block may leave
+                const int back = (stage + Shape::STAGES - first + i) % Shape::STAGES;
+                const unsigned round = (unsigned)((kb1 - kb0 - first + i) / Shape::STAGES) & 1;
+                if (!mbar_wait(&sh->empty[back], round)) { atomicExch(error_word, 2); break; }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(ROWS >> 3) << 17) | ((unsigned)(TR_BM >> 4) << 24);
+            int stage = 0;
+            unsigned phase = 0;
+            bool ok = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait(&sh->full[stage], phase)) { atomicExch(error_word, 4); ok = false; break; }
+                tc_fence_after();
+                const unsigned w_addr = smem_u32(ring + stage * Shape::STAGE_BYTES), x_addr = w_addr + TR_W_BYTES;
+#pragma unroll
+                for (int k = 0; k < TC_BK / 16; ++k)
+                    umma_bf16(tmem_base, umma_desc(w_addr + k * 32), umma_desc(x_addr + k * 32), idesc, (kb > kb0 || k) ? 1u : 0u);
+                umma_commit(&sh->empty[stage]);
+                if (++stage == Shape::STAGES) { stage = 0; phase ^= 1; }
+            }
+            if (ok) umma_commit(&sh->acc_full);
+        }
+    } else {
+        const int quarter = warp & 3;
+        if (mbar_wait(&sh->acc_full, 0)) {          // every stage has been read: the ring is free
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < ROWS / 32; ++c) {
+                float v[32];
+                __syncwarp();
+                tmem_load_32(tmem_base + ((unsigned)(quarter * 32) << 16) + c * 32, v);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) sums[(c * 32 + i) * TR_BM + quarter * 32 + lane] = v[i];
+            }
+            tc_fence_before();
+        } else if (lane == 0) {
+            atomicExch(error_word, 5);
+        }
+    }
+    __syncwarp();
+    qil_wait_for_producer();       // outputs are written below: what still reads them has ended
+    cluster_sync_all();
+    // 4 outputs of a row a thread, out of 4 sums, or of 4 of a gate and 4 of the matching up features (columns come as
+    // [8 gate, 8 up] groups); the cluster's blocks take rows in turn.  Everything an item needs is asked for before any of it
+    // is used, for U items at a time: what this costs is trips to other blocks' shared memory and to L2.
+    constexpr int GROUPS = PAIRS ? TR_BM / 8 : TR_BM / 4, PARTS = PAIRS ? 2 : 1, U = 4 / PARTS;
+    const int items = (M - (int)rank + (int)blocks - 1) / (int)blocks * GROUPS;
+    for (int item0 = threadIdx.x; item0 < items; item0 += 192 * U) {
+        float v[U][4 * PARTS];
+        uint2 rv[U];
+        int row[U], col[U];                    // the row, and the tile's column of the first sum
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int item = min(item0 + u * 192, items - 1), group = item % GROUPS;
+            row[u] = item / GROUPS * (int)blocks + (int)rank;
+            col[u] = PAIRS ? (group >> 1) * 16 + (group & 1) * 4 : group * 4;
+            rv[u] = make_uint2(0u, 0u);
+            if (!PAIRS && residual != nullptr && n0 + col[u] < N)
+                rv[u] = *reinterpret_cast<const uint2*>(residual + (size_t)row[u] * N + n0 + col[u]);
+#pragma unroll
+            for (int i = 0; i < 4 * PARTS; ++i) v[u][i] = 0.f;
+        }
+        for (unsigned b0 = 0; b0 < blocks; b0 += 4) {
+            float4 part[U][4][PARTS];
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int q = 0; q < PARTS; ++q)
+                        if (b0 + b < blocks) part[u][b][q] = cluster_read4(sums + row[u] * TR_BM + col[u] + q * 8, b0 + b);
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int q = 0; q < PARTS; ++q)
+                        if (b0 + b < blocks) {
+                            v[u][4 * q] += part[u][b][q].x; v[u][4 * q + 1] += part[u][b][q].y;
+                            v[u][4 * q + 2] += part[u][b][q].z; v[u][4 * q + 3] += part[u][b][q].w;
+                        }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int n = n0 + col[u];
+            if (item0 + u * 192 >= items || n >= N) continue;
+            uint2 packed;
+            bf16* o = reinterpret_cast<bf16*>(&packed);
+            if (PAIRS) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float gate = round_to<bf16>(v[u][i]), up = round_to<bf16>(v[u][4 * (PARTS - 1) + i]);
+                    const float act = round_to<bf16>(__fdividef(gate, 1.0f + __expf(-gate)));
+                    o[i] = __float2bfloat16_rn(act * up);
+                }
+                *reinterpret_cast<uint2*>(out + (size_t)row[u] * (N / 2) + n0 / 2 + (col[u] >> 4) * 8 + (col[u] & 4)) = packed;
+            } else {
+                const bf16* r4 = reinterpret_cast<const bf16*>(&rv[u]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float x = v[u][i];
+                    if (bias) x += __bfloat162float(bias[n + i]);
+                    if (residual) x = __bfloat162float(r4[i]) + x;
+                    o[i] = __float2bfloat16_rn(x);
+                }
+                *reinterpret_cast<uint2*>(out + (size_t)row[u] * N + n) = packed;
+            }
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();            // no block leaves while another reads its sums
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((unsigned)ROWS) : "memory");
+    }
+}
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -714,4 +929,68 @@ extern "C" int qil_gemm_tc_qkv(const void* a, const void* w, const void* bias, v
     tail.page_size = page_size > 0 ? page_size : 1; tail.num_pages = num_pages;
     const int N = (n_q_heads + 2 * n_kv_heads) * 128;
     return launch_gemm_tc(a, w, bias, nullptr, q_out, M, N, K, 0, sm_count, error_word, tail, stream);
+}
+
+// ------------------------------------------------------------------ a few dozen rows: launch
+template <int ROWS, bool PAIRS>
+static int launch_rows(const CUtensorMap& map_x, const CUtensorMap& map_w, const bf16* bias, const bf16* residual, bf16* out,
+                       int M, int N, int K, int blocks, int* error_word, cudaStream_t stream) {
+    const int smem = TrShape<ROWS>::SMEM;
+    static bool configured[64];                            // by device: the limit belongs to the function on a device
+    int device = -1;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess || device < 0 || device >= 64) QIL_REFUSE("gemm_tc_rows: device %d is out of range", device);
+    if (!configured[device]) {
+        e = cudaFuncSetAttribute(gemm_tc_rows_kernel<ROWS, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) QIL_REFUSE("gemm_tc_rows: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        configured[device] = true;
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((N + TR_BM - 1) / TR_BM * blocks);
+    config.blockDim = dim3(192);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = blocks;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = qil_chaining_enabled() ? 2 : 1;
+    e = cudaLaunchKernelEx(&config, gemm_tc_rows_kernel<ROWS, PAIRS>, map_x, map_w, bias, residual, out, M, N, K, error_word);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        snprintf(qil_error_text, sizeof(qil_error_text), "%s", cudaGetErrorString(e));
+        return (int)e;
+    }
+    QIL_CHECK_LAUNCH();
+}
+
+// M <= 128 rows; the rest as qil_gemm_tc.  Measured, us for a tile's K cut into 1 / 2 / 4 / 8 at 32 rows, weights from
+// memory: 6144 x 1024 9.3 / 6.5 / 8.0 / 14.9, 4096 x 4096 23.1 / 14.2 / 12.1 / 11.8, 6144 x 4096 23.5 / 15.3 / 14.2 / 20.1,
+// 1024 x 3072 18.2 / 10.9 / 7.7 / 6.8, 24576 x 4096 37.3 / 42.0 / 46 / 64: what a block adds up grows with the rows and the
+// cluster, so K is cut while a block keeps six stages and the blocks are at most four thirds of the SMs.
+extern "C" int qil_gemm_tc_rows(const void* a, const void* w, const void* bias, const void* residual, void* out,
+                                int M, int N, int K, int silu_pairs, int sm_count, int* error_word, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (M > 128) QIL_REFUSE("gemm_tc_rows: %d rows, 128 at most", M);
+    if (K <= 0 || K % 8) QIL_REFUSE("gemm_tc_rows: K %d must be a positive multiple of 8 (16-byte rows for TMA)", K);
+    if (N % 8) QIL_REFUSE("gemm_tc_rows: N %d must be a multiple of 8", N);
+    if (((uintptr_t)a | (uintptr_t)w | (uintptr_t)out | (uintptr_t)residual) & 15)
+        QIL_REFUSE("gemm_tc_rows: operands must be 16-byte aligned");
+    if (silu_pairs && (N % 16 || bias != nullptr || residual != nullptr))
+        QIL_REFUSE("gemm_tc_rows: silu_pairs needs N %% 16 == 0 and neither bias nor residual");
+    if (error_word == nullptr || sm_count <= 0) QIL_REFUSE("gemm_tc_rows: needs an error word and the SM count");
+    const int rows = M <= 32 ? 32 : M <= 64 ? 64 : 128, tiles = (N + TR_BM - 1) / TR_BM, k_blocks = (K + TC_BK - 1) / TC_BK;
+    int blocks = 1;
+    while (2 * blocks <= TR_MOST_BLOCKS && 6 * 2 * blocks <= k_blocks && tiles * 2 * blocks * 3 <= 4 * sm_count) blocks *= 2;
+    CUtensorMap map_x, map_w;
+    if (make_map(&map_x, a, M, K, rows)) return -1;
+    if (make_map(&map_w, w, N, K, TR_BM)) return -1;
+#define ROWS_ARGS map_x, map_w, (const bf16*)bias, (const bf16*)residual, (bf16*)out, M, N, K, blocks, error_word, stream
+    if (rows == 32) return silu_pairs ? launch_rows<32, true>(ROWS_ARGS) : launch_rows<32, false>(ROWS_ARGS);
+    if (rows == 64) return silu_pairs ? launch_rows<64, true>(ROWS_ARGS) : launch_rows<64, false>(ROWS_ARGS);
+    return silu_pairs ? launch_rows<128, true>(ROWS_ARGS) : launch_rows<128, false>(ROWS_ARGS);
+#undef ROWS_ARGS
 }

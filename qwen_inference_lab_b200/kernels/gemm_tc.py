@@ -79,6 +79,45 @@ def gemm_tc(a, weight, bias=None, residual=None, out=None, silu_pairs=False):
     return out
 
 
+ROWS_MOST = 128          # rows that ``gemm_rows`` takes
+
+
+def rows_usable(a, weight, silu_pairs=False) -> bool:
+    """Should ``gemm_rows`` take this product?  bfloat16, more rows than the decode product takes and not too many: see
+    ``tuning``."""
+    most = tuning.ROWS_PLAIN_MAX if not silu_pairs else tuning.ROWS_PAIRS_MAX if weight.shape[0] >= 148 * 128 else ROWS_MOST
+    return (a.shape[0] <= min(most, ROWS_MOST) and usable(a, weight) and weight.is_contiguous()
+            and (a.data_ptr() | weight.data_ptr()) % 16 == 0)
+
+
+def gemm_rows(a, weight, bias=None, residual=None, out=None, silu_pairs=False):
+    """``gemm_tc`` for at most 128 rows: the weights are streamed once, K cut over clusters of blocks."""
+    _need(a, "a", torch.bfloat16, 2); _need(weight, "weight", torch.bfloat16, 2)
+    m, k = a.shape
+    n = weight.shape[0]
+    if weight.shape[1] != k:
+        raise KernelError(f"gemm_rows: a {tuple(a.shape)} against weight {tuple(weight.shape)}")
+    out_shape = (m, n // 2) if silu_pairs else (m, n)
+    if bias is not None:
+        _need(bias, "bias", torch.bfloat16, 1)
+        if bias.shape[0] != n:
+            raise KernelError("gemm_rows: bias has the wrong length")
+    if residual is not None:
+        _need(residual, "residual", torch.bfloat16, 2)
+        if residual.shape != out_shape:
+            raise KernelError("gemm_rows: residual has the wrong shape")
+    if out is None:
+        out = torch.empty(out_shape, dtype=torch.bfloat16, device=a.device)
+    _need(out, "out", torch.bfloat16, 2)
+    if out.shape != out_shape:
+        raise KernelError("gemm_rows: out has the wrong shape")
+    word = error_word(a.device)
+    lib = library()
+    _check(lib, lib.qil_gemm_tc_rows(_p(a), _p(weight), _p(bias), _p(residual), _p(out), c_int(m), c_int(n), c_int(k),
+                                     c_int(1 if silu_pairs else 0), c_int(_sm_count), _p(word), _stream()), "gemm_rows")
+    return out
+
+
 QKV_TAIL_MIN_ROWS = tuning.QKV_TAIL_MIN_ROWS
 
 

@@ -32,6 +32,15 @@ SMALL_M_WIDE_MAX_ELEMENTS = _tuned("SMALL_M_WIDE_MAX_ELEMENTS", 1 << 28)
 #: From this many rows on the gate/up product runs on the tcgen05 tile kernel (the first row count the decode
 #: product does not take).
 TILE_KERNEL_MIN_ROWS = _tuned("TILE_KERNEL_MIN_ROWS", 17)
+#: Up to this many rows the streaming tcgen05 kernel (``gemm_tc.gemm_rows``) takes the gate/up product of a matrix of at
+#: least 148 tiles of 128 features, and any number up to its 128 of a smaller one (24576 x 4096 against the tile kernel:
+#: 38.9 / 41.0 us at 64 rows, 42.9 / 40.3 at 128; 6144 x 1024: 8.2 / 12.3 and 10.0 / 12.3).
+ROWS_PAIRS_MAX = _tuned("ROWS_PAIRS_MAX", 64)
+#: ... and every other product instead of the library's.  Alone the two are even (4096 x 4096 12.1 / 11.1 us at 32 rows, 4096 x
+#: 12288 22.9 / 23.5, 1024 x 2048 6.5 / 7.2); in a chain this one's start is hidden.  A recorded step of the 28-layer 1024-wide
+#: model with both, with gate/up alone and without: 1231 / 1252 / 1385 us at 17 rows, 1291 / 1391 / 1510 at 24, 1383 / 1419 / 1538 at
+#: 32, 1440 / 1418 / 1457 at 40; of the 36-layer 4096-wide one 3780 / 3871 / 3976, 3851 / 3951 / 4057, 4001 / 4022 / 4122, 4140 / 4073 / 4142.
+ROWS_PLAIN_MAX = _tuned("ROWS_PLAIN_MAX", 32)
 #: From this many rows on the q/k/v product runs on the tcgen05 kernels with its tail fused; below, the pair
 #: kernel has too few 256 x 256 tiles for the SM pairs and the library product plus the tail kernel win
 #: (6144 x 4096 at 2048 rows: 86 us against 75 + 24 us; at 256 rows the library wins).

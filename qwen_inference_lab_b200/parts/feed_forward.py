@@ -73,6 +73,8 @@ class GatedMLP(FeedForward):
             x = norm.forward(ctx, x)
         if self.pairs8 and ops.small_m_ok(x, self.gate_up._w):
             hidden = ops.gemm_small_m(x, self.gate_up._w, silu_pairs=True)
+        elif self.pairs8 and gemm_tc.rows_usable(x, self.gate_up._w, silu_pairs=True):
+            hidden = gemm_tc.gemm_rows(x, self.gate_up._w, silu_pairs=True)
         elif self.pairs8 and gemm_tc.usable(x, self.gate_up._w):
             # prompt portions: the tcgen05 kernel applies the activation in its epilogue, so the
             # [tokens, 2 * intermediate] product never goes to memory

@@ -13,7 +13,7 @@ from __future__ import annotations
 
 import torch
 
-from ..kernels import ops
+from ..kernels import gemm_tc, ops
 from .base import Param, Part
 
 
@@ -125,6 +125,9 @@ class Linear(Part):
                 if bias is not None:
                     result += bias.float()
                 return result
+            if gemm_tc.rows_usable(x, weight):
+                # the rows between a decode step's and a prompt portion's
+                return gemm_tc.gemm_rows(x, weight, bias=bias, residual=residual, out=out)
             if residual is not None and bias is None:
                 return torch.addmm(residual, x, weight.t(), out=out if out is not None else residual)
             if bias is not None:
