@@ -2,7 +2,7 @@
 // accumulation on the fifth-generation tensor cores: the projections of prompt
 // portions (M from a few dozen to thousands of tokens).
 //
-// Blackwell-native structure, one persistent block per SM, 192 threads:
+// Blackwell-native structure, one persistent block per SM, 320 threads:
 //   warp 0      one thread issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a
 //               128 x 64 tile of A and a 256 x 64 tile of W per stage into a 4-stage ring and
 //               arms the stage's mbarrier with the byte count;
@@ -10,8 +10,8 @@
 //               through matrix descriptors, accumulator in tensor memory) four times per stage,
 //               then tcgen05.commit, which frees the stage when the MMAs have read it; the warp
 //               also allocates and frees the 512 columns of tensor memory;
-//   warps 2-5   read the finished accumulator with tcgen05.ld (each warp its quarter of the 128
-//               lanes), apply the epilogue and store bfloat16; meanwhile warp 1 already fills
+//   warps 2-9   read the finished accumulator with tcgen05.ld (each warp its quarter of the 128
+//               lanes and one half of the columns), apply the epilogue and store bfloat16; meanwhile warp 1 already fills
 //               the other half of tensor memory with the next tile.
 // Tiles go round-robin over the blocks: tile = blockIdx.x + i * gridDim.x, tokens fastest, so
 // blocks that run together share the same weight columns in L2.
@@ -34,6 +34,8 @@ QIL_ERROR_STORAGE
 #define TC_BN 256
 #define TC_BK 64
 #define TC_STAGES 4
+#define TC_EPILOGUE_WARPS 8              // two a quarter of the lanes: half the time from the last MMA to the last store
+#define TC_THREADS (64 + 32 * TC_EPILOGUE_WARPS)
 #define TC_A_BYTES (TC_BM * TC_BK * 2)
 #define TC_B_BYTES (TC_BN * TC_BK * 2)
 #define TC_STAGE_BYTES (TC_A_BYTES + TC_B_BYTES)
@@ -227,12 +229,12 @@ __device__ __forceinline__ void tc_store_qkv_head(unsigned taddr, int m, int M, 
     }
 }
 
-// One warp's quarter (32 rows) of a finished 128 x 256 accumulator: tcgen05.ld 32 columns at a time,
-// epilogue, bfloat16 stores.  m is this lane's output row, n0 the tile's first output column.
+// One warp's quarter (32 rows) and half (128 columns) of a finished 128 x 256 accumulator: tcgen05.ld 32 columns at a time,
+// epilogue, bfloat16 stores.  m is this lane's output row, n0 its first output column.
 __device__ __forceinline__ void tc_store_accumulator(unsigned taddr, int m, int n0, int M, int N, int silu_pairs,
                                                      const bf16* __restrict__ bias, const bf16* residual, bf16* out) {
 #pragma unroll 1
-    for (int c = 0; c < TC_BN / 32; ++c) {
+    for (int c = 0; c < TC_BN / 64; ++c) {
         float v[32];
         __syncwarp();                              // the load below is a warp-wide instruction
         tmem_load_32(taddr + c * 32, v);
@@ -288,7 +290,7 @@ struct TcShared {
     unsigned pad;
 };
 
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const bf16* __restrict__ bias, const bf16* residual, bf16* out,
                int M, int N, int K, int silu_pairs, int* error_word, const TcQkvTail tail) {
@@ -302,7 +304,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < TC_STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&sh->acc_full[a], 1); mbar_init(&sh->acc_empty[a], 4); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&sh->acc_full[a], 1); mbar_init(&sh->acc_empty[a], TC_EPILOGUE_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {
@@ -319,6 +321,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_a) : "memory");
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_w) : "memory");
+            qil_wait_for_producer();
+            qil_release_consumer();      // the block holds its tensor memory
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -373,6 +377,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     } else {
         const int quarter = warp & 3;                      // the TMEM lanes this warp may read
+        const int half = warp < 6 ? 0 : 128;               // and the columns it takes
+        qil_wait_for_producer();                           // outputs may still be read, the residual written, before this
         int acc = 0;
         unsigned acc_phase = 0;
         bool ok = true;
@@ -381,13 +387,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (!mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; break; }
             tc_fence_after();
             const int m = m0 + quarter * 32 + lane;
-            const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * TC_BN;
+            const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * TC_BN + half;
             if (tail.q_out != nullptr) {
-#pragma unroll 1
-                for (int h = 0; h < TC_BN / 128; ++h)
-                    if (n0 + h * 128 < N) tc_store_qkv_head(taddr + h * 128, m, M, (n0 + h * 128) / 128, tail, bias);
+                if (n0 + half < N) tc_store_qkv_head(taddr, m, M, (n0 + half) / 128, tail, bias);
             } else {
-                tc_store_accumulator(taddr, m, n0, M, N, silu_pairs, bias, residual, out);
+                tc_store_accumulator(taddr, m, n0 + half, M, N, silu_pairs, bias, residual, out);
             }
             tc_fence_before();
             __syncwarp();
@@ -416,7 +420,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // Barriers.  full[s] lives in the first block: its producer arms it with the bytes of both blocks and
 // the second block's copies complete on it too (the barrier operand of a cta_group::2 copy may be the
 // peer's).  empty[s] and acc_full[a] exist in both blocks and are signalled by one tcgen05.commit with a
-// multicast mask of both.  acc_empty[a] lives in the first block and collects the arrivals of the eight
+// multicast mask of both.  acc_empty[a] lives in the first block and collects the arrivals of the sixteen
 // epilogue warps of the pair, the second block's through shared::cluster addresses.  Every wait is
 // local to the waiting block and bounded as in the kernel above; the pair meets at a cluster barrier
 // before either block frees its tensor memory and leaves.  None of the loads is a multicast load.
@@ -476,7 +480,7 @@ __device__ __forceinline__ unsigned umma_idesc_pair() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(256 >> 3) << 17) | ((unsigned)(256 >> 4) << 24);
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const bf16* __restrict__ bias, const bf16* residual, bf16* out,
                     int M, int N, int K, int silu_pairs, int* error_word, const TcQkvTail tail) {
@@ -492,7 +496,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < T2_STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&sh->acc_full[a], 1); mbar_init(&sh->acc_empty[a], 8); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&sh->acc_full[a], 1); mbar_init(&sh->acc_empty[a], 2 * TC_EPILOGUE_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {     // the same warp of both blocks, the same address: the pair's allocation
@@ -510,6 +514,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_a) : "memory");
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_w) : "memory");
+            qil_wait_for_producer();
+            qil_release_consumer();      // the block holds its tensor memory
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -559,7 +565,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else {
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, half = warp < 6 ? 0 : 128;
+        qil_wait_for_producer();
         int acc = 0;
         unsigned acc_phase = 0;
         bool ok = true;
@@ -568,13 +575,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; break; }
             tc_fence_after();
             const int m = m0 + quarter * 32 + lane;
-            const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * TC_BN;
+            const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * TC_BN + half;
             if (tail.q_out != nullptr) {
-#pragma unroll 1
-                for (int h = 0; h < TC_BN / 128; ++h)
-                    if (n0 + h * 128 < N) tc_store_qkv_head(taddr + h * 128, m, M, (n0 + h * 128) / 128, tail, bias);
+                if (n0 + half < N) tc_store_qkv_head(taddr, m, M, (n0 + half) / 128, tail, bias);
             } else {
-                tc_store_accumulator(taddr, m, n0, M, N, silu_pairs, bias, residual, out);
+                tc_store_accumulator(taddr, m, n0 + half, M, N, silu_pairs, bias, residual, out);
             }
             tc_fence_before();
             __syncwarp();
@@ -877,7 +882,7 @@ static int launch_gemm_tc(const void* a, const void* w, const void* bias, const 
             if (e != cudaSuccess) QIL_REFUSE("gemm_tc: cannot reserve %d bytes of shared memory: %s", smem_pair, cudaGetErrorString(e));
             cudaLaunchConfig_t config = {};
             config.gridDim = dim3(sm_count & ~1);
-            config.blockDim = dim3(192);
+            config.blockDim = dim3(TC_THREADS);
             config.dynamicSmemBytes = smem_pair;
             int clusters = 0;
             e = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel, &config);
@@ -886,14 +891,14 @@ static int launch_gemm_tc(const void* a, const void* w, const void* bias, const 
         }
         const int pair_tiles = ((M + 255) / 256) * ((N + TC_BN - 1) / TC_BN);
         const int pairs = pair_tiles < pairs_resident ? pair_tiles : pairs_resident;
-        gemm_tc_pair_kernel<<<2 * pairs, 192, smem_pair, stream>>>(map_a, map_w, (const bf16*)bias, (const bf16*)residual,
-                                                                   (bf16*)out, M, N, K, silu_pairs, error_word, tail);
+        qil_launch_chained(gemm_tc_pair_kernel, dim3(2 * pairs), dim3(TC_THREADS), smem_pair, stream, map_a, map_w, (const bf16*)bias,
+                           (const bf16*)residual, (bf16*)out, M, N, K, silu_pairs, error_word, tail);
         QIL_CHECK_LAUNCH();
     }
     const int n_tiles = ((M + TC_BM - 1) / TC_BM) * ((N + TC_BN - 1) / TC_BN);
     const int blocks = n_tiles < sm_count ? n_tiles : sm_count;
-    gemm_tc_kernel<<<blocks, 192, smem, stream>>>(map_a, map_w, (const bf16*)bias, (const bf16*)residual, (bf16*)out,
-                                                  M, N, K, silu_pairs, error_word, tail);
+    qil_launch_chained(gemm_tc_kernel, dim3(blocks), dim3(TC_THREADS), smem, stream, map_a, map_w, (const bf16*)bias,
+                       (const bf16*)residual, (bf16*)out, M, N, K, silu_pairs, error_word, tail);
     QIL_CHECK_LAUNCH();
 }
 
