@@ -82,12 +82,13 @@ def gemm_tc(a, weight, bias=None, residual=None, out=None, silu_pairs=False):
 ROWS_MOST = 128          # rows that ``gemm_rows`` takes
 
 
-def rows_usable(a, weight, silu_pairs=False) -> bool:
+def rows_usable(a, weight, silu_pairs=False, residual=None, out=None) -> bool:
     """Should ``gemm_rows`` take this product?  bfloat16, more rows than the decode product takes and not too many: see
-    ``tuning``."""
+    ``tuning``; whole rows on 16-byte boundaries."""
     most = tuning.ROWS_PLAIN_MAX if not silu_pairs else tuning.ROWS_PAIRS_MAX if weight.shape[0] >= 148 * 128 else ROWS_MOST
     return (a.shape[0] <= min(most, ROWS_MOST) and usable(a, weight) and weight.is_contiguous()
-            and (a.data_ptr() | weight.data_ptr()) % 16 == 0)
+            and (a.data_ptr() | weight.data_ptr()) % 16 == 0
+            and all(t is None or (t.is_contiguous() and t.data_ptr() % 16 == 0) for t in (residual, out)))
 
 
 def gemm_rows(a, weight, bias=None, residual=None, out=None, silu_pairs=False):

@@ -7,7 +7,7 @@ for its projections (qil/model.py:52-54,69-71: ``nn.Linear`` -> cuBLAS); every
 other combination (the true 32-bit path, or a weight stored in float32 inside a
 bfloat16 model) runs the engine's own float32 CUDA-core product.  Products of at
 most 16 rows (decode steps) run the engine's own weight-streaming kernel instead
-of the library.
+of the library, products of a few more its tcgen05 form (``gemm_tc.rows_usable``).
 """
 from __future__ import annotations
 
@@ -125,7 +125,7 @@ class Linear(Part):
                 if bias is not None:
                     result += bias.float()
                 return result
-            if gemm_tc.rows_usable(x, weight):
+            if gemm_tc.rows_usable(x, weight, residual=residual, out=out):
                 # the rows between a decode step's and a prompt portion's
                 return gemm_tc.gemm_rows(x, weight, bias=bias, residual=residual, out=out)
             if residual is not None and bias is None:
