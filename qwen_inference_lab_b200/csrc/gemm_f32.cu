@@ -4,9 +4,10 @@
 //
 // A row's result does not depend on which other rows share the launch: which kernel takes a product's rows depends on
 // how many they are, but all of them sum an element's products in one order.  float32 operands whose rows are whole
-// 16-byte vectors: K is cut into runs of `run_length(K)` (at most GEMM_RUNS of them), a run is two chains of FMA in
-// ascending k, one over its even and one over its odd k (a packed FMA works on both), whose sums are added; the runs'
-// sums are added in ascending order.  All other operands (`gemm_f32_kernel`): one chain over K in ascending k.
+// 16-byte vectors and longer than CHAIN_K: K is cut into runs of `run_length(K)` (at most GEMM_RUNS of them), a run is two
+// chains of FMA in ascending k, one over its even and one over its odd k (a packed FMA works on both), whose sums are
+// added; the runs' sums are added in ascending order.  All others: one chain over K in ascending k (a short K gains
+// little from being cut, and keeps the order that these products always had).
 //
 // Weights are row-major [out_features, in_features] as in the checkpoint
 // (qil/model.py:32-40: nn.Linear).
@@ -15,13 +16,32 @@
 // ---------------------------------------------------------------- float32 operands in whole vectors
 #define GEMM_RUNS 8
 #define RUN_STEP 32     // runs are multiples of this
+#define CHAIN_K 256     // up to here a product is one run and one chain
 
 static __host__ __device__ __forceinline__ int run_length(int K) {
+    if (K <= CHAIN_K) return CHAIN_K;
     return (((K + RUN_STEP - 1) / RUN_STEP + GEMM_RUNS - 1) / GEMM_RUNS) * RUN_STEP;
 }
 
 __device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// acc += the products of four k's: as two chains, or (CHAIN) as one, whose sum is the lower half of acc
+template <bool CHAIN>
+__device__ __forceinline__ void fma_quad(unsigned long long& acc, const ulonglong2& a, const ulonglong2& b) {
+    if (!CHAIN) {
+        fma_pair(acc, a.x, b.x);
+        fma_pair(acc, a.y, b.y);
+        return;
+    }
+    const float4 p = *reinterpret_cast<const float4*>(&a), q = *reinterpret_cast<const float4*>(&b);
+    float sum = __uint_as_float((unsigned)acc);
+    sum = fmaf(p.x, q.x, sum);
+    sum = fmaf(p.y, q.y, sum);
+    sum = fmaf(p.z, q.z, sum);
+    sum = fmaf(p.w, q.w, sum);
+    acc = __float_as_uint(sum);
 }
 
 __device__ __forceinline__ float pair_sum(unsigned long long v) {
@@ -77,7 +97,7 @@ __device__ __forceinline__ void gemm_store(const GemmArgs& g, int m, int n, floa
 #define STREAM_BK 32
 #define STREAM_LD (STREAM_BK + 4)      // a quarter warp's 16-byte reads of 8 rows meet every bank once
 
-template <int RM, int MG, int F>
+template <int RM, int MG, int F, bool CHAIN>
 __global__ void __launch_bounds__(STREAM_BN / F * MG)
 gemm_f32_stream_kernel(const GemmArgs g, int stages) {
     constexpr int MT = RM * MG, FT = STREAM_BN / F, THREADS = FT * MG;
@@ -144,10 +164,7 @@ gemm_f32_stream_kernel(const GemmArgs g, int stages) {
             for (int r = 0; r < RM; ++r) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + r * STREAM_BK + q * 4);
 #pragma unroll
-                for (int j = 0; j < F; ++j) {
-                    fma_pair(acc[j][r], a.x, w[j].x);
-                    fma_pair(acc[j][r], a.y, w[j].y);
-                }
+                for (int j = 0; j < F; ++j) fma_quad<CHAIN>(acc[j][r], a, w[j]);
             }
         }
         if ((s + 1) % run_stages == 0 || s + 1 == n_stages) {
@@ -194,7 +211,7 @@ gemm_f32_stream_kernel(const GemmArgs g, int stages) {
 #define TILE_LD (TILE_BK + 4)
 #define TILE_STAGES 2
 
-template <int BM>
+template <int BM, bool CHAIN>
 __global__ void __launch_bounds__(BM * 2, BM == 64 ? 3 : 6)
 gemm_f32_tile_kernel(const GemmArgs g) {
     constexpr int J = TILE_BN / 16, THREADS = BM * 2, TY = BM / 8, STAGE = (BM + TILE_BN) * TILE_LD;
@@ -260,6 +277,13 @@ gemm_f32_tile_kernel(const GemmArgs g) {
 #pragma unroll
         for (int q = 0; q < TILE_BK / 4; ++q) {
             if (q + 1 < TILE_BK / 4) read(q + 1);
+            if (CHAIN) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < J; ++j) fma_quad<true>(acc[i][j], a[q & 1][i], w[q & 1][j]);
+                continue;
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -404,7 +428,8 @@ static cudaError_t launch_stream(const GemmArgs& g, int blocks, int stages, cuda
     const int tiles = (g.N + STREAM_BN - 1) / STREAM_BN;
     size_t smem = (size_t)stages * (STREAM_BN * STREAM_LD + RM * MG * STREAM_BK) * sizeof(float);
     if (blocks > 1) smem += (size_t)(GEMM_RUNS / blocks) * RM * MG * STREAM_BN * sizeof(float);
-    return launch_clusters(gemm_f32_stream_kernel<RM, MG, F>, dim3(tiles * blocks), STREAM_BN / F * MG, smem, blocks, stream, g, stages);
+    return launch_clusters(g.K > CHAIN_K ? gemm_f32_stream_kernel<RM, MG, F, false> : gemm_f32_stream_kernel<RM, MG, F, true>,
+                           dim3(tiles * blocks), STREAM_BN / F * MG, smem, blocks, stream, g, stages);
 }
 
 template <int BM_>
@@ -412,7 +437,7 @@ static cudaError_t launch_tile(const GemmArgs& g, int blocks, cudaStream_t strea
     const size_t ring = (size_t)TILE_STAGES * (BM_ + TILE_BN) * TILE_LD * sizeof(float);
     const size_t sums = (size_t)BM_ * TILE_BN * sizeof(float);
     const dim3 grid((g.N + TILE_BN - 1) / TILE_BN * blocks, (g.M + BM_ - 1) / BM_);
-    return launch_clusters(gemm_f32_tile_kernel<BM_>, grid, BM_ * 2, blocks > 1 ? (ring > sums ? ring : sums) : ring + sums,
+    return launch_clusters(g.K > CHAIN_K ? gemm_f32_tile_kernel<BM_, false> : gemm_f32_tile_kernel<BM_, true>, grid, BM_ * 2, blocks > 1 ? (ring > sums ? ring : sums) : ring + sums,
                            blocks, stream, g);
 }
 
@@ -432,9 +457,10 @@ static double tile_waves(long long count) {
 //   1024 237 / 253: a cluster costs a quarter on top and pays where its finer blocks fill the SMs better than that.
 static cudaError_t gemm_f32_vectors(const GemmArgs& g, cudaStream_t stream) {
     const long long columns = (g.N + 63) / 64;             // STREAM_BN and TILE_BN
+    const bool chain = g.K <= CHAIN_K;                     // one run: nothing for a cluster to share
     if (g.M <= 16) {
         int blocks = 1;
-        while (blocks < GEMM_RUNS && columns * blocks < 5 * 148) blocks *= 2;
+        while (!chain && blocks < GEMM_RUNS && columns * blocks < 5 * 148) blocks *= 2;
         const int stages = columns * blocks <= 2 * 148 ? 8 : 4;        // few blocks: a deeper ring in each
         if (g.M <= 1) return launch_stream<1, 1, 1>(g, blocks, stages, stream);
         if (g.M <= 2) return launch_stream<2, 1, 1>(g, blocks, stages, stream);
@@ -442,9 +468,9 @@ static cudaError_t gemm_f32_vectors(const GemmArgs& g, cudaStream_t stream) {
         if (g.M <= 8) return launch_stream<4, 2, 1>(g, blocks, stages, stream);
         return launch_stream<4, 4, 2>(g, blocks, stages, stream);
     }
-    if (g.M <= 64) return launch_tile<32>(g, columns * ((g.M + 31) / 32) < 6 * 148 ? GEMM_RUNS : 1, stream);
+    if (g.M <= 64) return launch_tile<32>(g, !chain && columns * ((g.M + 31) / 32) < 6 * 148 ? GEMM_RUNS : 1, stream);
     const long long tiles = columns * ((g.M + 63) / 64);
-    return launch_tile<64>(g, tile_waves(tiles) * GEMM_RUNS > 1.25 * tile_waves(tiles * GEMM_RUNS) ? GEMM_RUNS : 1, stream);
+    return launch_tile<64>(g, !chain && tile_waves(tiles) * GEMM_RUNS > 1.25 * tile_waves(tiles * GEMM_RUNS) ? GEMM_RUNS : 1, stream);
 }
 
 // residual may alias C (each element is read and written by the same thread).
