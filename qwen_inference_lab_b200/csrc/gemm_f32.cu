@@ -91,8 +91,8 @@ __device__ __forceinline__ void gemm_store(const GemmArgs& g, int m, int n, floa
 // streams 64 weight rows through a ring of stages of 32 k (one 128-byte line a row and stage); a thread holds one
 // F features and RM rows, MG groups of 64 / F threads share a stage.  Bound by memory at one row (151936 x 1024: 105 us,
 // 5.9 TB/s), from eight on by the shared-memory reads of the activations, which broadcast to a warp (143 us; a thread of
-// twice the rows or features has too few warps beside it).  The 64 x 64 tiles this replaced took 8 rows like 64: 4096 x
-// 1024 in 190 us, now 10.
+// twice the rows or features has too few warps beside it).  The 64 x 64 tiles this replaced took 8 rows like 64: a decode
+// step of 8 rows of the 1024-wide model 68.3 ms, 36.9 with this alone.
 #define STREAM_BN 64
 #define STREAM_BK 32
 #define STREAM_LD (STREAM_BK + 4)      // a quarter warp's 16-byte reads of 8 rows meet every bank once
@@ -453,7 +453,7 @@ static double tile_waves(long long count) {
 //   16.0 / 11.6; 1 row 151936 x 1024 105 / 138 / 109 / 144.  So a cluster as large as fills five blocks an SM.
 //   16 rows with the stream kernel 10.5 and 14.7 (4096 x 1024, 1024 x 3072), 24 with 32-row tiles 18.1 and 22.3.
 //   32-row tiles against 64-row tiles: 64 rows 28.4 / 31.3 and 27.6 / 34.3; 128 rows the wider ones halve the weight reads.
-//   64-row tiles alone and in clusters of eight: 128 x 4096 x 1024 64.5 / 49.7, 512 x 1024 x 3072 173 / 123, 512 x 6144 x
+//   64-row tiles (with stages of 16 k) alone and in clusters of eight: 128 x 4096 x 1024 64.5 / 49.7, 512 x 1024 x 3072 173 / 123, 512 x 6144 x
 //   1024 237 / 253: a cluster costs a quarter on top and pays where its finer blocks fill the SMs better than that.
 static cudaError_t gemm_f32_vectors(const GemmArgs& g, cudaStream_t stream) {
     const long long columns = (g.N + 63) / 64;             // STREAM_BN and TILE_BN
