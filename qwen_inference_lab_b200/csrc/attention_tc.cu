@@ -459,12 +459,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
             const float sum = (sums[0] + sums[1]) + (sums[2] + sums[3]);
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j + 3);
-            if (__any_sync(0xffffffffu, factor != 1.0f)) {
+            const bool rescale = __any_sync(0xffffffffu, factor != 1.0f);
+            if (rescale || (j > 0 && j == n_tiles - 1)) {
                 // O may be touched once the previous tile's second MMA is done.  (P needs no such wait: it goes
-                // over this tile's own scores.  The barrier is at most one phase ahead of the awaited one, as
-                // the next second MMA cannot be issued before this warp has published P.)
+                // over this tile's own scores.)  Before P is published the barrier can be in two phases only, the awaited
+                // one or the next: these scores followed the second MMA of two tiles ago, and this tile's own
+                // second MMA waits for this warp.  After it, it could also be a phase behind (another warp still at its
+                // rescale of the tile before), which the parity of the last wait below cannot tell from done: so the
+                // last tile waits here whether it rescales or not.  Its second MMA follows the awaited one anyway.
                 if (!at_wait(&sh->pv_done, (j - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 22); ok = false; break; }
                 at_fence_after();
+            }
+            if (rescale) {
 #pragma unroll 1
                 for (int c = 0; c < (AT_E + 31) / 32; ++c) {
                     unsigned r[32];
