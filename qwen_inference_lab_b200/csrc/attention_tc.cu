@@ -381,6 +381,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const bool biased = p.slopes_log2 != nullptr;
         const float slope = biased ? p.slopes_log2[head] : 0.f;
         const float scale_later = (biased || capped) ? 1.0f : p.scale_log2;
+        // A tile of fewer than 128 tokens moves its maximum whenever it grows, as the 64-token kernel (attention_mma.cu)
+        // that would take it does: a largest weight of exactly 1 has no rounding, and with the slack the error against 64
+        // bits was up to 1.07 of that kernel's.
+        const float slack = (rows < AT_M && row < rows) ? 0.f : 8.f;
         float m_used = -INFINITY, l = 0.f;
         bool ok = true;
         for (int j = 0; j < n_tiles && ok; ++j) {
@@ -435,9 +439,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 mx[2] = fmaxf(mx[2], s[i + 2]); mx[3] = fmaxf(mx[3], s[i + 3]);
             }
             const float tmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_later;
-            // Move the maximum only when it grew by more than 2^8: until then exp2(s - m_used) <= 256,
+            // Move the maximum only when it grew by more than 2^8 (`slack`): until then exp2(s - m_used) <= 256,
             // harmless in float32 and bfloat16, and O needs no rescale (which costs a TMEM round trip).
-            const bool grow = tmax > m_used + 8.0f;            // also true at the first tile (m_used = -inf)
+            const bool grow = tmax > m_used + slack;           // also true at the first tile (m_used = -inf)
             const float factor = (grow && j > 0) ? at_exp2(m_used - tmax) : 1.0f;
             if (grow) m_used = tmax;
             const float minus_m = (m_used == -INFINITY) ? 0.f : -m_used;

@@ -23,10 +23,15 @@ QUERY_TILE = 64          # tokens per query tile of ``attn_prefill_kernel``
 BIG_QUERY_TILE = attention_tc.TILE     # tokens per query tile of the tensor-memory kernel
 
 
-#: A tail's context from which on the tensor-memory kernel takes it whatever its length.  It walks a context at 1 us per
-#: 64 keys, the 64-token kernel at 2.2, and has a launch less when nothing is left to the other one; what it wastes is
-#: rows of a tile.  Measured on 32 heads of 128: a tail of 125 tokens behind 1920, 70 us of a kernel of its own against
-#: none beside three whole tiles.
+#: A tail's context from which on the tensor-memory kernel takes it whatever its length.  It walks a context at 0.8 us per
+#: 64 keys, the 64-token kernel at 2, and has a launch less when nothing is left to the other one; what it wastes is
+#: rows of a tile.  Measured (us, L2 flushed before each, 64-token kernel / tensor-memory kernel; 32 heads of 128 over 8):
+#:   one tail of 2 tokens behind 200, 300, 1024, 4096, 16384     12 / 10, 14 / 10, 38 / 21, 135 / 57, 522 / 201
+#:   one tail of 100                                             16 / 11, 20 / 14, 40 / 24, 135 / 68, 518 / 224
+#:   16 tails of 2 behind 200, 300, 1024, 4096                   30 / 23, 35 / 24, 92 / 52, 328 / 147
+#:   16 tails of 100                                             60 / 28, 74 / 35, 164 / 63, 533 / 179
+#: It loses up to 1.5 us where both take little: 65 to 127 tokens behind nothing (7.5 / 8.5 for one of 65 and 8.1 / 8.5 for
+#: one of 100; 16 of 100: 28 / 20), heads of 64 and 32 behind 300 (9 / 9 and 8 / 8, 16 tails of 2 of the latter 10 / 11).
 TAIL_CONTEXT = 256
 
 

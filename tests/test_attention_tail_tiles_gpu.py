@@ -50,3 +50,23 @@ def test_every_token_is_in_one_tile():
     for token, _, _, _ in plan["decode_info"].reshape(-1, 4):
         seen[token] += 1
     assert (seen == 1).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,length,start", [(128, 700, 663), (128, 1500, 1391), (64, 900, 898), (32, 400, 335)])
+def test_a_tail_is_as_exact_as_in_the_64_token_kernel(d, length, start):
+    # which kernel takes a segment's tail is a matter of time alone: the error of its tiles may not be larger.  Both round
+    # the weights and the result to bfloat16 at the same places, so the errors of some 10^5 values agree to a per cent
+    from qwen_inference_lab_b200.kernels import attention_mma, attention_tc
+    q, pool, table, meta, expected = attention_case(16, 4, d, [length, length + 64], [start, start + 64], torch.bfloat16, 16, seed=3)
+    q, pool, table = q.cuda(), pool.cuda(), table.cuda()
+    def tiles(size):
+        info = [v for first, n, pos0, row in zip(meta["seg_start"], meta["seg_len"], meta["seg_pos0"], meta["seg_row"])
+                for off in range(0, n, size) for v in (first + off, pos0 + off, min(size, n - off), row)]
+        return torch.tensor(info, dtype=torch.int32).cuda(), len(info) // 4
+    by_64, by_128 = torch.empty_like(q), torch.empty_like(q)
+    attention_mma.prefill(q, pool, by_64, *tiles(64), table, 16, 4, d, 16, 0, d ** -0.5)
+    attention_tc.prefill(q, pool, by_128, *tiles(128), table, 16, 4, 16, d ** -0.5, head_dim=d)
+    error = lambda out: float((out.cpu().double() - expected.double()).norm() / expected.double().norm())
+    assert error(by_128) <= 1.01 * error(by_64)
+    attention_tc.check()
