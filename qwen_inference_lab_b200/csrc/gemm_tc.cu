@@ -20,7 +20,8 @@
 // [8 gate rows, 8 up rows] and the kernel writes silu(gate) * up, N/2 values per token
 // (qil/model.py:71), so the [M, 2I] intermediate never exists in memory.
 //
-// Every wait on an mbarrier is bounded.  A wait that runs out records its place in the error
+// Every wait on an mbarrier is bounded (and begins once the kernel before this one has ended: launched chained, a block may
+// be there long before).  A wait that runs out records its place in the error
 // word, the role stops issuing, every role runs out in turn, the producer drains its copies in
 // flight (again bounded), the tensor memory is freed and the kernel returns; the host reads the
 // error word.  No multicast loads are used.
@@ -348,6 +349,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     } else if (warp == 1) {
         if (lane == 0) {
             const unsigned idesc = umma_idesc();
+            qil_wait_for_producer();       // the bounded waits below count this kernel's own time
             int stage = 0, acc = 0;
             unsigned phase = 0, acc_phase = 0;
             bool ok = true;
@@ -539,6 +541,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             const unsigned idesc = umma_idesc_pair();
+            qil_wait_for_producer();
             int stage = 0, acc = 0;
             unsigned phase = 0, acc_phase = 0;
             bool ok = true;
@@ -702,6 +705,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     } else if (warp == 1) {
         if (lane == 0) {
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(ROWS >> 3) << 17) | ((unsigned)(TR_BM >> 4) << 24);
+            qil_wait_for_producer();       // the rows come after it; the bounded waits count this kernel's own time
             int stage = 0;
             unsigned phase = 0;
             bool ok = true;
@@ -719,6 +723,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         }
     } else {
         const int quarter = warp & 3;
+        qil_wait_for_producer();
         if (mbar_wait(&sh->acc_full, 0)) {          // every stage has been read: the ring is free
             tc_fence_after();
 #pragma unroll 1

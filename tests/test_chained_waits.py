@@ -1,0 +1,40 @@
+"""Kernels that are launched chained begin while the kernel before them still runs: how long that takes may not count
+against their bounded waits."""
+import re
+from pathlib import Path
+
+import pytest
+
+SOURCE = (Path(__file__).resolve().parent.parent / "qwen_inference_lab_b200" / "csrc" / "gemm_tc.cu").read_text()
+KERNELS = ("gemm_tc_kernel", "gemm_tc_pair_kernel", "gemm_tc_rows_kernel")
+
+
+def block(text, at):
+    """The text between the brace at or after ``at`` and its partner, and where it ends."""
+    begin = text.index("{", at)
+    depth = 0
+    for i in range(begin, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[begin + 1:i], i + 1
+    raise AssertionError("unbalanced braces")
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_every_role_waits_for_the_kernel_before_ahead_of_its_first_bounded_wait(kernel):
+    source = re.sub(r"//[^\n]*", "", SOURCE)
+    definition = re.search(r"__global__[^;{]*?\b%s\(" % kernel, source)
+    assert re.search(r"qil_launch_chained\(%s|cudaLaunchKernelEx\(&config, %s" % (kernel, kernel), source)
+    body, _ = block(source, source.index(")", definition.end()))
+    at, roles = body.index("if (warp == 0) {"), []
+    while True:
+        role, end = block(body, at)
+        roles.append(role)
+        follows = re.match(r"\s*else\b", body[end:])
+        if not follows:
+            break
+        at = end
+    assert len(roles) == 3                                 # loads, MMAs, epilogue
+    for role in roles:
+        assert "mbar_wait(" in role
+        assert role.split("mbar_wait(")[0].count("qil_wait_for_producer();") == 1, role[:200]
