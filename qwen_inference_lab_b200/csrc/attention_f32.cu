@@ -249,7 +249,7 @@ attention_f32_single_kernel(const float* __restrict__ q, const Pages pages, floa
         for (int s = 0; s < n_spans; ++s) {
             const float2 v = __ldcg(reinterpret_cast<const float2*>(part_ml) + slot + s);
             const float o = __ldcg(part_o + (slot + s) * D + d);
-            if (v.x == -INFINITY) continue;
+            if (v.y == 0.f) continue;           // no key was seen (weights that are not a number do count)
             const float2 f = join(m_run, l_run, v.x, v.y);
             o_run = fmaf(o_run, f.x, __fmul_rn(o, f.y));
         }
@@ -446,7 +446,7 @@ attention_f32_tile_kernel(const float* __restrict__ q, const Pages pages, float*
         for (int r = 0; r < PER; ++r) {
             if (row0 + r >= rows) continue;
             const float m = ml[2 * (row0 + r)], l = ml[2 * (row0 + r) + 1];
-            if (m == -INFINITY) continue;
+            if (l == 0.f) continue;             // no key was seen (weights that are not a number do count)
             const float2 f = join(m_run[r], l_run[r], m, l), a = pair_of(acc[r][0]), b = pair_of(acc[r][1]);
             o_run[r][0] = fmaf(o_run[r][0], f.x, __fmul_rn(a.x, f.y));
             o_run[r][1] = fmaf(o_run[r][1], f.x, __fmul_rn(a.y, f.y));

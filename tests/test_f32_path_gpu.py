@@ -76,3 +76,41 @@ def test_attention_f32(case):
     positions, token_row = flat_meta(meta)
     ops.attention_generic(q, pool, generic, positions, token_row, table, n_q, n_kv, d, page, window, d ** -0.5)
     torch.testing.assert_close(tiled, generic, atol=2e-6, rtol=2e-5)
+
+
+def both_kernels(q, pool, table, info, n_q, n_kv, d, page, window=0):
+    """The same tokens (first, position, row) through the tile kernel, the span kernel and the general one."""
+    from qwen_inference_lab_b200.kernels import attention_f32, ops
+    as_int = lambda values: torch.tensor(values, dtype=torch.int32).cuda()
+    shape = (table, n_q, n_kv, d, page, window, d ** -0.5)
+    tiled, alone, generic = (torch.full_like(q, 7.0) for _ in range(3))
+    n, n_spans = len(info), max(pos for _, pos, _ in info) // 256 + 1
+    attention_f32.tiles(q, pool, tiled, as_int([v for at, pos, row in info for v in (at, pos, 1, row)]), n, *shape)
+    scratch = (torch.empty(n * n_q * n_spans * d, device="cuda"), torch.empty(n * n_q * n_spans * 2, device="cuda"),
+               torch.zeros(n * n_kv, dtype=torch.int32, device="cuda"))
+    attention_f32.singles(q, pool, alone, as_int([v for at, pos, row in info for v in (at, pos, row, 0)]), n, n_spans, scratch, *shape)
+    ops.attention_generic(q, pool, generic, as_int([pos for _, pos, _ in info]), as_int([row for _, _, row in info]), *shape)
+    return tiled, alone, generic
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")], ids=["nan", "inf", "minus_inf"])
+@pytest.mark.parametrize("place", ["key", "value"])
+def test_attention_f32_of_what_is_no_number(place, bad):
+    """A key or a value that is not finite: seen, it shows as in the general kernel (a key alone in its span too); unseen
+    (behind the token, before the window, in an unused slot), it does not."""
+    n_q, n_kv, d, page, length = 4, 2, 64, 16, 600
+    generator = torch.Generator().manual_seed(8)
+    pool = torch.randn(length // page + 1, 2, n_kv, page, d, generator=generator)
+    at = 512                                             # the first key of the third span
+    column = slice(None) if place == "key" and bad != bad else 0
+    pool[at // page, 0 if place == "key" else 1, :, at % page, column] = bad
+    table = torch.arange(length // page + 1, dtype=torch.int32).view(1, -1).cuda()
+    positions = [10, 255, 511, 512, 513, 599]
+    q = torch.randn(len(positions), n_q * d, generator=generator).cuda()
+    for window in (0, 90, 1):
+        tiled, alone, generic = both_kernels(q, pool.cuda(), table, [(i, pos, 0) for i, pos in enumerate(positions)], n_q, n_kv, d, page, window)
+        torch.testing.assert_close(tiled, generic, atol=2e-6, rtol=2e-5, equal_nan=True)
+        torch.testing.assert_close(alone, tiled, atol=0.0, rtol=0.0, equal_nan=True)
+        for i, pos in enumerate(positions):
+            seen = at <= pos and not (window and pos - window + 1 > at)
+            assert seen or bool(torch.isfinite(tiled[i]).all())
