@@ -14,8 +14,10 @@ SPAN = 256                       # keys a span, the same number as in the source
 HEAD_DIMS = (32, 64, 128)
 MOST_GROUP = 64                  # query heads per kv head of the tile kernel: its rows
 MOST_SINGLE_GROUP = 8            # ... of the span kernel
-#: Bytes of partial sums the span kernel may have.  They are sized by the longest context times the tokens: beyond this
-#: (64 tokens of 32 heads of 128 reach it at 65536 positions) a block walks its token's spans itself, which takes none.
+#: Bytes of partial sums the span kernel's buffer may have.  They are sized by the longest context times the tokens: beyond
+#: this (64 tokens of 32 heads of 128 reach it at 65536 positions) a block walks its token's spans itself, which takes
+#: none and is slower (64 tokens of 32 heads of 128 over 8 at 16384 positions: 10.1 ms against 1.9).  Recorded graphs keep
+#: the buffer that they were recorded with, so the smaller ones it grew from may stay beside it.
 MOST_SCRATCH = 256 << 20
 
 
@@ -64,5 +66,5 @@ def attend(ctx, q, cache, out, n_q_heads, n_kv_heads, head_dim, window, scale):
         if n_q_heads // n_kv_heads > MOST_SINGLE_GROUP or 4 * n_single * n_q_heads * n_spans * head_dim > MOST_SCRATCH:
             tiles(q, cache.pages, out, arrays["decode_info"], n_single, *shape, singles=True)
         else:
-            scratch = attention_mma.decode_scratch(ctx, n_single, n_q_heads, n_spans, head_dim)
+            scratch = attention_mma.decode_scratch(ctx, n_single, n_q_heads, n_spans, head_dim, most=MOST_SCRATCH)
             singles(q, cache.pages, out, arrays["decode_info"], n_single, n_spans, scratch, *shape)

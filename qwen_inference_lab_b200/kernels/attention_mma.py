@@ -199,22 +199,24 @@ def merge_in_kernel(n_decode, n_q_heads, n_kv_heads, head_dim) -> bool:
     return blocks_per_span <= int(os.environ.get("QIL_TICKET_MAX_BLOCKS", _slots(head_dim)))
 
 
-def decode_scratch(ctx, n_decode, n_q_heads, n_spans, head_dim):
+def decode_scratch(ctx, n_decode, n_q_heads, n_spans, head_dim, most=None):
     """Partial sums, their (max, sum) pairs and the ticket counters for the single-token kernel (the blocks
     of a token's spans count themselves in, the last one merges; the counters are zero between launches).
 
     One pair of buffers per runner, kept in ``ctx.extras`` (which the runner carries from step to
     step) and replaced by a larger pair when a step needs more; a recorded graph keeps the pair it
-    was recorded with alive.
+    was recorded with alive.  ``most``: bytes of partial sums up to which a larger pair is made with room to grow.
     """
     slots = n_decode * n_q_heads * n_spans
     scratch = ctx.extras.get("attn_decode_scratch")
     # one counter per (token, kv head, chunk of 16 query heads) at most: a counter per query head is always enough
     if scratch is None or scratch[0].numel() < slots * head_dim or scratch[1].numel() < slots * 2 \
             or len(scratch) < 3 or scratch[2].numel() < n_decode * n_q_heads:
-        grow = lambda old, need: max(need, 2 * old.numel() if old is not None else 0)
+        def grow(old, need, limit=None):
+            room = 2 * old.numel() if old is not None else 0
+            return max(need, room if limit is None else min(room, limit))
         old = (tuple(scratch) + (None, None, None))[:3] if scratch else (None, None, None)
-        scratch = (torch.empty(grow(old[0], slots * head_dim), dtype=torch.float32, device=ctx.device),
+        scratch = (torch.empty(grow(old[0], slots * head_dim, most and most // 4), dtype=torch.float32, device=ctx.device),
                    torch.empty(grow(old[1], slots * 2), dtype=torch.float32, device=ctx.device),
                    torch.zeros(grow(old[2], n_decode * n_q_heads), dtype=torch.int32, device=ctx.device))
         ctx.extras["attn_decode_scratch"] = scratch
