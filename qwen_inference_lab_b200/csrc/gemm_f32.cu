@@ -484,6 +484,7 @@ extern "C" int qil_gemm_f32(const void* A, int lda, const void* Wt, const void* 
         const GemmArgs g = {(const float*)A, (const float*)Wt, (const float*)bias, (const float*)residual, (float*)C, col_scale, M, N, K, lda};
         const cudaError_t e = gemm_f32_vectors(g, stream);
         if (e != cudaSuccess) {
+            cudaGetLastError();             // reported here: the next launch does not answer for it
             snprintf(qil_error_text, sizeof(qil_error_text), "%s", cudaGetErrorString(e));
             return (int)e;
         }

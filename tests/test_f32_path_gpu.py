@@ -114,3 +114,25 @@ def test_attention_f32_of_what_is_no_number(place, bad):
         for i, pos in enumerate(positions):
             seen = at <= pos and not (window and pos - window + 1 > at)
             assert seen or bool(torch.isfinite(tiled[i]).all())
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """A product on a stream whose recording has been broken fails on the host; the next kernel does not answer for it."""
+    from qwen_inference_lab_b200.kernels import ops
+    from qwen_inference_lab_b200.kernels.ops import KernelError
+    a, w, x, gain = (torch.ones(*shape, device="cuda") for shape in ((4, 512), (64, 512), (3, 64), (64,)))
+    out, normed = torch.empty(4, 64, device="cuda"), torch.empty(3, 64, device="cuda")
+    ops.gemm_f32(a, w, out=out)
+    ops.rmsnorm(x, gain, 1e-6, out=normed)
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="thread_local")
+        with pytest.raises(RuntimeError):
+            stream.synchronize()                               # not while it records: the recording is broken from here on
+        with pytest.raises(KernelError):
+            ops.gemm_f32(a, w, out=out)
+        with pytest.raises(RuntimeError):
+            graph.capture_end()
+    ops.rmsnorm(x, gain, 1e-6, out=normed)
+    torch.testing.assert_close(normed, torch.ones_like(normed))
