@@ -271,7 +271,7 @@ class StepRunner:
         """Raise if a kernel of an earlier step reported a fault of its own (a bounded wait that ran
         out).  Kernels with such reports register them with ``ops.register_post_step_check``.  A check
         costs nothing unless its kernel was launched since the last one; then it waits for the device,
-        or with ``wait=False`` reports a step or two late instead (``ops.ErrorWord``)."""
+        or with ``wait=False`` reports a step or two late instead (of replayed steps some more: ``ops.ErrorWord``)."""
         ops.run_post_step_checks(wait)
 
     def _run_graph(self, description):
@@ -321,17 +321,20 @@ class StepRunner:
                     current.capture_begin(**mode)
 
                 try:
-                    logits = self.model.forward(ctx, self.views, logit_rows, checkpoint=cut)
+                    with ops.marks() as words:
+                        logits = self.model.forward(ctx, self.views, logit_rows, checkpoint=cut)
                 finally:
                     current.capture_end()
                 graphs.append(current)
             torch.cuda.current_stream().wait_stream(stream)
             # the graphs hold addresses of what the parts keep in ``extras`` (scratch): keep those alive
-            self._graphs[key] = (graphs, logits, launches, dict(self._extras))
+            self._graphs[key] = (graphs, logits, launches, words, dict(self._extras))
             self.launches_per_graph[n] = launches
             self.kernel_launches += launches
             return eager_logits
-        graphs, logits, launches = record[:3]
+        graphs, logits, launches, words = record[:4]
+        for word in words:
+            word.mark(replayed=True)
         for graph in graphs:
             graph.replay()
         self.kernel_launches += launches
