@@ -6,8 +6,7 @@
 // how many they are, but all of them sum an element's products in one order.  float32 operands whose rows are whole
 // 16-byte vectors and longer than CHAIN_K: K is cut into runs of `run_length(K)` (at most GEMM_RUNS of them), a run is two
 // chains of FMA in ascending k, one over its even and one over its odd k (a packed FMA works on both), whose sums are
-// added; the runs' sums are added in ascending order.  All others: one chain over K in ascending k (a short K gains
-// little from being cut, and keeps the order that these products always had).
+// added; the runs' sums are added in ascending order.  All others: one chain over K in ascending k.
 //
 // Weights are row-major [out_features, in_features] as in the checkpoint
 // (qil/model.py:32-40: nn.Linear).
@@ -16,7 +15,12 @@
 // ---------------------------------------------------------------- float32 operands in whole vectors
 #define GEMM_RUNS 8
 #define RUN_STEP 32     // runs are multiples of this
-#define CHAIN_K 256     // up to here a product is one run and one chain
+// Up to here a product is one run and one chain in ascending k, as in the kernel below that took all of them once.  That
+// order is neither faster nor closer to the exact sum than runs are (a step of five rows of a 96-wide model: 71 us with
+// runs of 32, 76 with 64, 85 with 128, 96 with the chain).  It is kept for float32 models that are held to an oracle in
+// float32: a replayed row of a small Virulix model is compared at 1e-5 (1 + |x|) with an oracle that is itself 1.01e-5 from
+// 64 bits there, and left that tolerance (1.17e-5) with runs of 32, 64 and 128 and with the chain up to a K of 80 only.
+#define CHAIN_K 256
 
 static __host__ __device__ __forceinline__ int run_length(int K) {
     if (K <= CHAIN_K) return CHAIN_K;
@@ -88,8 +92,8 @@ __device__ __forceinline__ void gemm_store(const GemmArgs& g, int m, int n, floa
 }
 
 // Up to 16 rows (a decode step): the weights are read once and everything else has to stay out of their way.  A block
-// streams 64 weight rows through a ring of stages of 32 k (one 128-byte line a row and stage); a thread holds one
-// F features and RM rows, MG groups of 64 / F threads share a stage.  Bound by memory at one row (151936 x 1024: 105 us,
+// streams 64 weight rows through a ring of stages of 32 k (one 128-byte line a row and stage); a thread holds F
+// features and RM rows, MG groups of 64 / F threads share a stage.  Bound by memory at one row (151936 x 1024: 105 us,
 // 5.9 TB/s), from eight on by the shared-memory reads of the activations, which broadcast to a warp (143 us; a thread of
 // twice the rows or features has too few warps beside it).  The 64 x 64 tiles this replaced took 8 rows like 64: a decode
 // step of 8 rows of the 1024-wide model 68.3 ms, 36.9 with this alone.
@@ -99,7 +103,7 @@ __device__ __forceinline__ void gemm_store(const GemmArgs& g, int m, int n, floa
 
 template <int RM, int MG, int F, bool CHAIN>
 __global__ void __launch_bounds__(STREAM_BN / F * MG)
-gemm_f32_stream_kernel(const GemmArgs g, int stages) {
+gemm_f32_stream_kernel(const GemmArgs g, int stages) {      // stages: 4 or 8
     constexpr int MT = RM * MG, FT = STREAM_BN / F, THREADS = FT * MG;
     constexpr int STAGE = STREAM_BN * STREAM_LD + MT * STREAM_BK;
     extern __shared__ __align__(16) float smem[];
@@ -150,7 +154,7 @@ gemm_f32_stream_kernel(const GemmArgs g, int stages) {
         for (int r = 0; r < RM; ++r) { acc[j][r] = 0ull; total[j][r] = 0.f; }
     for (int s = 0; s < n_stages; ++s) {
         // the oldest of the groups in flight is this stage
-        if (stages == 4) copies_wait<2>(); else if (stages == 8) copies_wait<6>(); else copies_wait<0>();
+        if (stages == 4) copies_wait<2>(); else copies_wait<6>();
         __syncthreads();
         load(s + stages - 1);
         const float* ws = smem + s % stages * STAGE + f * STREAM_LD;
@@ -277,21 +281,21 @@ gemm_f32_tile_kernel(const GemmArgs g) {
 #pragma unroll
         for (int q = 0; q < TILE_BK / 4; ++q) {
             if (q + 1 < TILE_BK / 4) read(q + 1);
-            if (CHAIN) {
+            if constexpr (CHAIN) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
 #pragma unroll
                     for (int j = 0; j < J; ++j) fma_quad<true>(acc[i][j], a[q & 1][i], w[q & 1][j]);
-                continue;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a[q & 1][i].x, w[q & 1][j].x);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a[q & 1][i].y, w[q & 1][j].y);
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a[q & 1][i].x, w[q & 1][j].x);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < J; ++j) fma_pair(acc[i][j], a[q & 1][i].y, w[q & 1][j].y);
         }
         if (blocks == 1 && ((s + 1) % run_stages == 0 || s + 1 == n_stages)) {
             const bool first = s < run_stages, last = s + 1 == n_stages;
