@@ -11,9 +11,6 @@
 
 #define SPAN 256
 
-__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
 __device__ __forceinline__ float2 pair_of(unsigned long long v) {
     float2 f;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
@@ -24,14 +21,6 @@ __device__ __forceinline__ unsigned long long twice(float v) {
     asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(v));
     return p;
 }
-__device__ __forceinline__ void copy16(float* to, const float* from, bool inside) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(to);
-    const int bytes = inside ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(from), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
-
 struct Pages {
     const float* cache;
     const int* block_table;

@@ -74,6 +74,64 @@ static inline cudaError_t qil_launch_chained(void (*kernel)(KArgs...), dim3 grid
     return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
 }
 
+// The same as clusters of `blocks` blocks along x.
+template <typename... KArgs, typename... Args>
+static inline cudaError_t qil_launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int blocks,
+                                              cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = blocks;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = qil_chaining_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
+}
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_blocks() {
+    unsigned n;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;\n" : "=r"(n));
+    return n;
+}
+// The shared::cluster address of the same shared-memory offset in block `rank` of the cluster.
+__device__ __forceinline__ unsigned map_to_rank(unsigned shared_addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(shared_addr), "r"(rank));
+    return r;
+}
+// Every thread of every block of the cluster meets here; shared memory written before is visible after.
+__device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// 16 bytes from global to shared memory; zeros when the vector lies outside the operand (`from` then only has to be a
+// valid address)
+__device__ __forceinline__ void copy16(float* to, const float* from, bool inside) {
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(to);
+    const int bytes = inside ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
+
+// Two float32 FMA in one instruction, each rounded by itself.
+__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<bf16>(bf16 v) { return __bfloat162float(v); }

@@ -27,10 +27,6 @@ static __host__ __device__ __forceinline__ int run_length(int K) {
     return (((K + RUN_STEP - 1) / RUN_STEP + GEMM_RUNS - 1) / GEMM_RUNS) * RUN_STEP;
 }
 
-__device__ __forceinline__ void fma_pair(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-
 // acc += the products of four k's: as two chains, or (CHAIN) as one, whose sum is the lower half of acc
 template <bool CHAIN>
 __device__ __forceinline__ void fma_quad(unsigned long long& acc, const ulonglong2& a, const ulonglong2& b) {
@@ -54,27 +50,10 @@ __device__ __forceinline__ float pair_sum(unsigned long long v) {
     return lo + hi;
 }
 
-// 16 bytes from global to shared memory; zeros when the vector lies outside the operand (`from` then only has to be a
-// valid address)
-__device__ __forceinline__ void copy16(float* to, const float* from, bool inside) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(to);
-    const int bytes = inside ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(from), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int LEFT> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
-
 // Blocks of a cluster share a tile's runs: block r of c takes runs r * GEMM_RUNS / c on.
-__device__ __forceinline__ void cluster_barrier() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
 __device__ __forceinline__ float cluster_read(const float* at, int rank) {
-    const unsigned mine = (unsigned)__cvta_generic_to_shared(at);
-    unsigned theirs;
     float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(theirs) : "memory");
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_rank((unsigned)__cvta_generic_to_shared(at), rank)) : "memory");
     return v;
 }
 
@@ -108,9 +87,7 @@ gemm_f32_stream_kernel(const GemmArgs g, int stages) {      // stages: 4 or 8
     constexpr int STAGE = STREAM_BN * STREAM_LD + MT * STREAM_BK;
     extern __shared__ __align__(16) float smem[];
     float* sums = smem + stages * STAGE;                 // [runs of this block][MT][STREAM_BN]
-    unsigned blocks, rank;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(blocks));
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const unsigned blocks = cluster_blocks(), rank = cluster_rank();
     const int tid = threadIdx.x, f = tid % FT, mg = tid / FT;
     const int n0 = blockIdx.x / blocks * STREAM_BN;
     const int run = run_length(g.K), runs = (g.K + run - 1) / run, per = GEMM_RUNS / blocks;
@@ -193,14 +170,14 @@ gemm_f32_stream_kernel(const GemmArgs g, int stages) {      // stages: 4 or 8
             }
         return;
     }
-    cluster_barrier();
+    cluster_sync_all();
     for (int e = rank * THREADS + tid; e < g.M * STREAM_BN; e += blocks * THREADS) {
         if (n0 + e % STREAM_BN >= g.N) continue;
         float v = 0.f;
         for (int r = 0; r < runs; ++r) v += cluster_read(sums + r % per * MT * STREAM_BN + e, r / per);
         gemm_store(g, e / STREAM_BN, n0 + e % STREAM_BN, v);
     }
-    cluster_barrier();      // no block leaves while another reads its sums
+    cluster_sync_all();      // no block leaves while another reads its sums
 }
 
 // More rows: 8 x 4 outputs a thread, tiles of BM x 64, both operands through a ring of stages of 32 k as they lie in
@@ -220,9 +197,7 @@ __global__ void __launch_bounds__(BM * 2, BM == 64 ? 3 : 6)
 gemm_f32_tile_kernel(const GemmArgs g) {
     constexpr int J = TILE_BN / 16, THREADS = BM * 2, TY = BM / 8, STAGE = (BM + TILE_BN) * TILE_LD;
     extern __shared__ __align__(16) float smem[];
-    unsigned blocks, rank;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(blocks));
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const unsigned blocks = cluster_blocks(), rank = cluster_rank();
     // one block: its running sums beside the ring; a cluster: the run's sums in the ring's place
     float* sums = blocks > 1 ? smem : smem + TILE_STAGES * STAGE;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -325,7 +300,7 @@ gemm_f32_tile_kernel(const GemmArgs g) {
 #pragma unroll
             for (int j = 0; j < J; ++j) sums[(ty + i * TY) * TILE_BN + tx + j * 16] = pair_sum(acc[i][j]);
     }
-    cluster_barrier();
+    cluster_sync_all();
     for (int e = rank * THREADS + tid; e < BM * TILE_BN; e += blocks * THREADS) {
         const int m = m0 + e / TILE_BN, n = n0 + e % TILE_BN;
         if (m >= g.M || n >= g.N) continue;
@@ -333,7 +308,7 @@ gemm_f32_tile_kernel(const GemmArgs g) {
         for (int r = 0; r < runs; ++r) v += cluster_read(sums + e, r);
         gemm_store(g, m, n, v);
     }
-    cluster_barrier();
+    cluster_sync_all();
 }
 
 // ---------------------------------------------------------------- any types, any K
@@ -411,20 +386,7 @@ static cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, int thre
                                    cudaStream_t stream, Args... args) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t config = {};
-    config.gridDim = grid;
-    config.blockDim = dim3(threads);
-    config.dynamicSmemBytes = smem;
-    config.stream = stream;
-    cudaLaunchAttribute attributes[2];
-    attributes[0].id = cudaLaunchAttributeClusterDimension;
-    attributes[0].val.clusterDim.x = blocks;
-    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
-    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attributes[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attributes;
-    config.numAttrs = qil_chaining_enabled() ? 2 : 1;
-    return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
+    return qil_launch_clusters(kernel, grid, dim3(threads), smem, blocks, stream, args...);
 }
 
 template <int RM, int MG, int F>

@@ -440,21 +440,6 @@ struct Tc2Shared {
     unsigned pad;
 };
 
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-// The shared::cluster address of the same shared-memory offset in block `rank` of the cluster.
-__device__ __forceinline__ unsigned map_to_rank(unsigned shared_addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(shared_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
 __device__ __forceinline__ void mbar_arrive_cluster(unsigned cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }
@@ -652,9 +637,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     TrShared* sh = reinterpret_cast<TrShared*>(ring + Shape::STAGES * Shape::STAGE_BYTES);
     float* sums = reinterpret_cast<float*>(ring);          // [ROWS][128] once the ring is read out
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned rank = cluster_rank();
-    unsigned blocks;
-    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(blocks));
+    const unsigned rank = cluster_rank(), blocks = cluster_blocks();
     const int n0 = blockIdx.x / blocks * TR_BM;
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
     const int kb0 = (int)((long long)k_blocks * rank / blocks), kb1 = (int)((long long)k_blocks * (rank + 1) / blocks);
@@ -955,20 +938,8 @@ static int launch_rows(const CUtensorMap& map_x, const CUtensorMap& map_w, const
         if (e != cudaSuccess) QIL_REFUSE("gemm_tc_rows: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
         configured[device] = true;
     }
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((N + TR_BM - 1) / TR_BM * blocks);
-    config.blockDim = dim3(192);
-    config.dynamicSmemBytes = smem;
-    config.stream = stream;
-    cudaLaunchAttribute attributes[2];
-    attributes[0].id = cudaLaunchAttributeClusterDimension;
-    attributes[0].val.clusterDim.x = blocks;
-    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
-    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attributes[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attributes;
-    config.numAttrs = qil_chaining_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&config, gemm_tc_rows_kernel<ROWS, PAIRS>, map_x, map_w, bias, residual, out, M, N, K, error_word);
+    e = qil_launch_clusters(gemm_tc_rows_kernel<ROWS, PAIRS>, dim3((N + TR_BM - 1) / TR_BM * blocks), dim3(192), smem, blocks, stream,
+                            map_x, map_w, bias, residual, out, M, N, K, error_word);
     if (e != cudaSuccess) {
         cudaGetLastError();
         snprintf(qil_error_text, sizeof(qil_error_text), "%s", cudaGetErrorString(e));
