@@ -70,3 +70,62 @@ def test_a_tail_is_as_exact_as_in_the_64_token_kernel(d, length, start):
     error = lambda out: float((out.cpu().double() - expected.double()).norm() / expected.double().norm())
     assert error(by_128) <= 1.01 * error(by_64)
     attention_tc.check()
+
+
+OPTIONS = {
+    # d, v_dim, window, and what else the scores get
+    "slopes": (64, 64, 0, dict(slopes=True)),
+    "cap": (128, 128, 0, dict(softcap=4.0)),
+    "cap_and_slopes": (32, 32, 0, dict(softcap=3.0, slopes=True)),
+    "chunk": (64, 64, 0, dict(chunk=150)),
+    "sink": (128, 128, 0, dict(sink=True)),
+    "chunk_cap_sink": (64, 64, 0, dict(chunk=96, softcap=5.0, sink=True)),
+    "window_and_slopes": (64, 64, 90, dict(slopes=True)),
+    "wide_values": (16, 64, 0, dict()),
+    "narrow_values": (128, 64, 0, dict(sink=True)),
+    "values_window": (48, 80, 70, dict(slopes=True)),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", OPTIONS)
+def test_tiles_of_fewer_tokens_with_every_score_option(name):
+    """Tails of 1 to 127 tokens behind contexts in and out of step with key tiles and chunks, unused slots full of NaN, beside
+    the general kernel (float32 arithmetic on the same bfloat16 operands)."""
+    from qwen_inference_lab_b200.kernels import attention_tc, ops
+    d, v_dim, window, options = OPTIONS[name]
+    n_q, n_kv, page = 8, 2, 16
+    segments = [(0, 1), (63, 2), (64, 127), (149, 65), (300, 37), (511, 3), (700, 100)]          # (position, tokens)
+    generator = torch.Generator().manual_seed(sum(map(ord, name)))
+    draw = lambda *shape: torch.randn(*shape, generator=generator)
+    pages, table = [], torch.full((len(segments), 60), -1, dtype=torch.int32)
+    for row, (start, count) in enumerate(segments):
+        for at in range(0, start + count, page):
+            keys, values = draw(n_kv, page, d), draw(n_kv, page, v_dim)
+            keys[:, max(0, start + count - at):] = values[:, max(0, start + count - at):] = float("nan")
+            table[row, at // page] = len(pages)
+            pages.append(torch.cat([keys.reshape(-1), values.reshape(-1)]))
+    pages = torch.stack(pages).bfloat16().cuda()
+    if v_dim == d:
+        pages = pages.view(-1, 2, n_kv, page, d)
+    table = table.cuda()
+    q = draw(sum(count for _, count in segments), n_q * d).bfloat16().cuda()
+    info, positions, rows = [], [], []
+    for row, (start, count) in enumerate(segments):
+        info += [len(positions), start, count, row]
+        positions += range(start, start + count)
+        rows += [row] * count
+    as_int = lambda values: torch.tensor(values, dtype=torch.int32).cuda()
+    slopes = (0.02 * torch.arange(1, n_q + 1)).cuda() if options.get("slopes") else None
+    sinks = draw(n_q).cuda() if options.get("sink") else None
+    softcap, chunk = options.get("softcap", 0.0), options.get("chunk", 0)
+    log2e = 1.4426950408889634
+    out = torch.full((q.shape[0], n_q * v_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    attention_tc.prefill(q, pages, out, as_int(info), len(segments), table, n_q, n_kv, page, d ** -0.5,
+                         slopes_log2=None if slopes is None else slopes * log2e, chunk=chunk,
+                         sink_log2=None if sinks is None else sinks * log2e, softcap=softcap, window=window, head_dim=d, v_dim=v_dim)
+    attention_tc.check()
+    expected = torch.empty_like(out)
+    ops.attention_generic(q, pages, expected, as_int(positions), as_int(rows), table, n_q, n_kv, d, page, window, d ** -0.5,
+                          v_dim=v_dim, slopes=slopes, softcap=softcap, chunk=chunk, sink_logits=sinks)
+    close(out, expected.float(), torch.bfloat16, scale=2)
