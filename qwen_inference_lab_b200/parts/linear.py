@@ -130,10 +130,11 @@ class Linear(Part):
                 return gemm_tc.gemm_rows(x, weight, bias=bias, residual=residual, out=out)
             if residual is not None and bias is None:
                 return torch.addmm(residual, x, weight.t(), out=out if out is not None else residual)
-            if bias is not None:
-                result = torch.addmm(bias, x, weight.t(), out=out)
-            else:
-                result = torch.mm(x, weight.t(), out=out) if out is not None else torch.mm(x, weight.t())
+            if bias is None:
+                return torch.mm(x, weight.t(), out=out) if out is not None else torch.mm(x, weight.t())
+            if residual is not None and out is not None and out.data_ptr() == residual.data_ptr():
+                return ops.add_inplace(out, torch.addmm(bias, x, weight.t()))       # the residual outlasts the product
+            result = torch.addmm(bias, x, weight.t(), out=out)
             if residual is not None:
                 ops.add_inplace(result, residual)
             return result
