@@ -411,7 +411,7 @@ def attend(ctx, q, cache, out, n_q_heads, n_kv_heads, head_dim, window, scale, s
                                         ("tile_info", "big_tile_info", "rest_tile_info", "decode_info"))
     if n_big and (not options or attention_tc.takes(options)) and not shared_rows \
             and attention_tc.supports(head_dim, cache.page_size, window, v_dim):
-        # whole 128-token tiles on tcgen05 with the accumulators in tensor memory, the leftovers below
+        # tiles of up to 128 tokens on tcgen05 with the accumulators in tensor memory, the leftovers below
         if options:
             options.check(n_q_heads)
         attention_tc.prefill(q, cache.pages, out, arrays["big_tile_info"], n_big, cache.block_table,

@@ -1,7 +1,7 @@
-"""The tcgen05/TMA attention for whole 128-token query tiles (bfloat16, head and value sizes up to 128), compiled per pair of
-sizes on first use.
+"""The tcgen05/TMA attention for query tiles of up to 128 tokens (bfloat16, head and value sizes up to 128), compiled per pair
+of sizes on first use.
 
-``prefill`` takes tiles of exactly 128 tokens; :func:`attention_mma.prefill` takes what is left.
+``prefill`` takes the tiles that ``attention_mma.describe_segments`` cuts for it; :func:`attention_mma.prefill` takes what is left.
 The kernel's mbarrier waits are bounded and report through an error word that ``check()`` reads.
 """
 from __future__ import annotations

@@ -29,17 +29,21 @@ SMALL_M_LIBRARY_ELEMENTS = _tuned("SMALL_M_LIBRARY_ELEMENTS", 1 << 28)
 #: its fewer instructions per weight byte (6144 x 4096 with the norm: 20.3 -> 18.5 us; 24576 x 4096: 37.2 -> 36.2).
 SMALL_M_WIDE_MIN_BLOCKS = _tuned("SMALL_M_WIDE_MIN_BLOCKS", 148)
 SMALL_M_WIDE_MAX_ELEMENTS = _tuned("SMALL_M_WIDE_MAX_ELEMENTS", 1 << 28)
-#: From this many rows on the gate/up product runs on the tcgen05 tile kernel (the first row count the decode
-#: product does not take).
+#: From this many rows on the gate/up product runs on the tcgen05 kernels (the first row count the decode product does not
+#: take): the streaming one up to the limits below, from there on the tile kernel.
 TILE_KERNEL_MIN_ROWS = _tuned("TILE_KERNEL_MIN_ROWS", 17)
 #: Up to this many rows the streaming tcgen05 kernel (``gemm_tc.gemm_rows``) takes the gate/up product of a matrix of at
 #: least 148 tiles of 128 features, and any number up to its 128 of a smaller one (24576 x 4096 against the tile kernel:
-#: 38.9 / 41.0 us at 64 rows, 42.9 / 40.3 at 128; 6144 x 1024: 8.2 / 12.3 and 10.0 / 12.3).
+#: 38.9 / 41.0 us at 64 rows, 42.9 / 40.3 at 128; 6144 x 1024: 8.2 / 12.3 and 10.0 / 12.3).  Where K is cut over a cluster the
+#: sums come in another order than the tile kernel's; against 64 bits both are as far off (12 shapes of K 96 to 25600, 17 to 128
+#: rows, 3 seeds each: relative errors of 3.50e-3 to 3.65e-3, ratio 0.996 to 1.003 either way).
 ROWS_PAIRS_MAX = _tuned("ROWS_PAIRS_MAX", 64)
 #: ... and every other product instead of the library's.  Alone the two are even (4096 x 4096 12.1 / 11.1 us at 32 rows, 4096 x
 #: 12288 22.9 / 23.5, 1024 x 2048 6.5 / 7.2); in a chain this one's start is hidden.  A recorded step of the 28-layer 1024-wide
 #: model with both, with gate/up alone and without: 1231 / 1252 / 1385 us at 17 rows, 1291 / 1391 / 1510 at 24, 1383 / 1419 / 1538 at
 #: 32, 1440 / 1418 / 1457 at 40; of the 36-layer 4096-wide one 3780 / 3871 / 3976, 3851 / 3951 / 4057, 4001 / 4022 / 4122, 4140 / 4073 / 4142.
+#: (The kernel itself takes up to 128 rows here too, for whoever raises the line.)  Against 64 bits a plain product is as far
+#: off as the library's (1.66e-3), one with a residual less (1.66e-3 against 2.15e-3: one rounding instead of two).
 ROWS_PLAIN_MAX = _tuned("ROWS_PLAIN_MAX", 32)
 #: From this many rows on the q/k/v product runs on the tcgen05 kernels with its tail fused; below, the pair
 #: kernel has too few 256 x 256 tiles for the SM pairs and the library product plus the tail kernel win
