@@ -1,8 +1,10 @@
 // Causal grouped-query attention over the paged cache for any head size, page
 // size and dtype, on the CUDA cores with float32 arithmetic throughout.
 //
-// This is the attention of the true 32-bit path, and the one that serves head
-// sizes or dtypes the tensor-core kernels do not take.  One block computes one
+// This is the attention that serves what the others do not take: float32 heads of
+// other sizes than 32, 64 and 128 or with any of the options below
+// (attention_f32.cu has the rest of the true 32-bit path), and head sizes or
+// dtypes beyond the tensor-core kernels.  One block computes one
 // (token, query head): scores against the keys of its request from the window's
 // start to the token's own position (absolute positions, so a chunk that
 // continues a cached prefix is masked correctly; qil/model.py:62-64), softmax

@@ -18,7 +18,7 @@
 //               second MMA takes its first operand from there: no shared memory, no proxy fence),
 //               and the rescale of O in tensor memory when the running maximum moved by more than
 //               2^8 (until then P is computed against the older maximum, which is exact algebra and
-//               safe in float32); finally O / l -> global memory.
+//               safe in float32), in tiles of fewer tokens whenever it moved; finally O / l -> global memory.
 // K tiles are K-major operands and V tiles MN-major operands of the same shared-memory image
 // ([key][64 elements = 128 bytes] x the slabs of the head).
 //

@@ -948,7 +948,8 @@ static int launch_rows(const CUtensorMap& map_x, const CUtensorMap& map_w, const
     QIL_CHECK_LAUNCH();
 }
 
-// M <= 128 rows; the rest as qil_gemm_tc.  Measured, us for a tile's K cut into 1 / 2 / 4 / 8 at 32 rows, weights from
+// M <= 128 rows; the rest as qil_gemm_tc.  (Products without silu_pairs come with up to 32 rows unless the caller's line is raised:
+// from 40 on the library's are faster in a step.)  Measured, us for a tile's K cut into 1 / 2 / 4 / 8 at 32 rows, weights from
 // memory: 6144 x 1024 9.3 / 6.5 / 8.0 / 14.9, 4096 x 4096 23.1 / 14.2 / 12.1 / 11.8, 6144 x 4096 23.5 / 15.3 / 14.2 / 20.1,
 // 1024 x 3072 18.2 / 10.9 / 7.7 / 6.8, 24576 x 4096 37.3 / 42.0 / 46 / 64: what a block adds up grows with the rows and the
 // cluster, so K is cut while a block keeps six stages and the blocks are at most four thirds of the SMs.
