@@ -24,7 +24,7 @@ def block(text, at):
 def test_every_role_waits_for_the_kernel_before_ahead_of_its_first_bounded_wait(kernel):
     source = re.sub(r"//[^\n]*", "", SOURCE)
     definition = re.search(r"__global__[^;{]*?\b%s\(" % kernel, source)
-    assert re.search(r"qil_launch_chained\(%s|cudaLaunchKernelEx\(&config, %s" % (kernel, kernel), source)
+    assert re.search(r"qil_launch_(chained|clusters)\(%s\b" % kernel, source)
     body, _ = block(source, source.index(")", definition.end()))
     at, roles = body.index("if (warp == 0) {"), []
     while True:
