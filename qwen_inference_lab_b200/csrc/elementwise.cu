@@ -92,23 +92,27 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const W* __restrict__ we
 
 // bfloat16 rows of up to 256 * 8 * RMS_VPT elements: the whole row sits in registers, every load is
 // 16 bytes wide and issued before the first use, so a row costs one memory round trip, not one per element.
+// TPR threads take a row: 256 of them, or a warp one of up to 1024, which needs no barrier, and a block of a step of many rows
+// eight of those (2920 rows of 1024: 7.9 -> 4.0 us).  128 threads a row of 4096 instead of 256: 2048 rows 9.6 -> 9.1 us, but 64 rows
+// 3.0 -> 3.8, which is what a decode step has.
 #define RMS_VPT 4
-template <typename W>
+template <typename W, int TPR>
 __global__ void __launch_bounds__(256)
 rmsnorm_bf16x8_kernel(const bf16* __restrict__ x, const W* __restrict__ weight, const int* __restrict__ rows,
-                      bf16* __restrict__ out, int width, float eps) {
-    __shared__ float scratch[32];
+                      bf16* __restrict__ out, int n_rows, int width, float eps) {
+    __shared__ float scratch[8];
     qil_wait_for_producer();
     qil_release_consumer();
-    const int r = blockIdx.x;
-    const int src_row = rows ? rows[r] : r;
+    const int tid = threadIdx.x % TPR, r = blockIdx.x * (blockDim.x / TPR) + threadIdx.x / TPR;
+    const bool live = r < n_rows;                 // uniform over a row's threads
+    const int src_row = !live ? 0 : rows ? rows[r] : r;
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)src_row * width);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)r * width);
-    const int vectors = width / 8;
+    const int vectors = live ? width / 8 : 0;
     uint4 v[RMS_VPT];
 #pragma unroll
     for (int i = 0; i < RMS_VPT; ++i) {
-        const int idx = threadIdx.x + i * 256;
+        const int idx = tid + i * TPR;
         v[i] = idx < vectors ? src[idx] : make_uint4(0u, 0u, 0u, 0u);
     }
     float sq = 0.f;
@@ -118,11 +122,19 @@ rmsnorm_bf16x8_kernel(const bf16* __restrict__ x, const W* __restrict__ weight, 
 #pragma unroll
         for (int k = 0; k < 8; ++k) { const float f = __bfloat162float(e[k]); sq += f * f; }
     }
-    sq = block_sum(sq, scratch);
+    sq = warp_sum(sq);
+    if (TPR > 32) {                               // the row's warps, in their order
+        const int warp = threadIdx.x >> 5, first = warp / (TPR / 32) * (TPR / 32);
+        if ((threadIdx.x & 31) == 0) scratch[warp] = sq;
+        __syncthreads();
+        sq = scratch[first];
+#pragma unroll
+        for (int i = 1; i < TPR / 32; ++i) sq += scratch[first + i];
+    }
     const float scale = 1.0f / sqrtf(sq / (float)width + eps);
 #pragma unroll
     for (int i = 0; i < RMS_VPT; ++i) {
-        const int idx = threadIdx.x + i * 256;
+        const int idx = tid + i * TPR;
         if (idx >= vectors) continue;
         uint4 o4;
         if (sizeof(W) == 2) {
@@ -180,6 +192,16 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const float* __restrict__ weight
     }
 }
 
+template <typename W>
+static void rmsnorm_bf16x8(const bf16* x, const W* weight, const int* rows, bf16* out, int n_rows, int width, float eps, cudaStream_t stream) {
+    auto launch = [&](auto kernel, int tpr) {
+        const int per_block = n_rows > 4 * 148 ? 256 / tpr : 1;       // few rows: a block each, on as many SMs
+        qil_launch_chained(kernel, dim3((n_rows + per_block - 1) / per_block), dim3(tpr * per_block), 0, stream, x, weight, rows, out, n_rows, width, eps);
+    };
+    if (width <= 32 * 8 * RMS_VPT) launch(rmsnorm_bf16x8_kernel<W, 32>, 32);
+    else launch(rmsnorm_bf16x8_kernel<W, 256>, 256);
+}
+
 extern "C" int qil_rmsnorm(const void* x, const void* weight, const int* rows, void* out,
                            int n_rows, int width, float eps, int act_dtype, int weight_dtype,
                            cudaStream_t stream) {
@@ -187,12 +209,8 @@ extern "C" int qil_rmsnorm(const void* x, const void* weight, const int* rows, v
     if (width <= 0) QIL_REFUSE("rmsnorm: width %d", width);
     if (act_dtype == QIL_BF16 && width % 8 == 0 && width <= 256 * 8 * RMS_VPT &&
         (((uintptr_t)x | (uintptr_t)out | (uintptr_t)weight) & 15) == 0) {
-        if (weight_dtype == QIL_BF16)
-            qil_launch_chained(rmsnorm_bf16x8_kernel<bf16>, dim3(n_rows), dim3(256), 0, stream,
-                               (const bf16*)x, (const bf16*)weight, rows, (bf16*)out, width, eps);
-        else if (weight_dtype == QIL_F32)
-            qil_launch_chained(rmsnorm_bf16x8_kernel<float>, dim3(n_rows), dim3(256), 0, stream,
-                               (const bf16*)x, (const float*)weight, rows, (bf16*)out, width, eps);
+        if (weight_dtype == QIL_BF16) rmsnorm_bf16x8((const bf16*)x, (const bf16*)weight, rows, (bf16*)out, n_rows, width, eps, stream);
+        else if (weight_dtype == QIL_F32) rmsnorm_bf16x8((const bf16*)x, (const float*)weight, rows, (bf16*)out, n_rows, width, eps, stream);
         else QIL_REFUSE("unknown dtype code %d", weight_dtype);
         QIL_CHECK_LAUNCH();
     }
