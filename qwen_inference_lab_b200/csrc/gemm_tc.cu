@@ -25,8 +25,7 @@
 // word, the role stops issuing, every role runs out in turn, the producer drains its copies in
 // flight (again bounded), the tensor memory is freed and the kernel returns; the host reads the
 // error word.  No multicast loads are used.
-#include "common.cuh"
-#include <cuda.h>
+#include "tcgen05.cuh"
 #include <stdlib.h>
 
 QIL_ERROR_STORAGE
@@ -40,93 +39,6 @@ QIL_ERROR_STORAGE
 #define TC_A_BYTES (TC_BM * TC_BK * 2)
 #define TC_B_BYTES (TC_BN * TC_BK * 2)
 #define TC_STAGE_BYTES (TC_A_BYTES + TC_B_BYTES)
-#define TC_WAIT_CYCLES 2000000000ll      // about a second
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-    unsigned done;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}\n"
-                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
-// Bounded wait: false when the barrier did not complete in about a second.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long start = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (clock64() - start > TC_WAIT_CYCLES) return false;
-    }
-    return true;
-}
-
-__device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
-                 ::"r"(smem_u32(smem)), "l"((unsigned long long)map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
-}
-
-// The same with the hint that these bytes are the first to leave L2: a weight tile that only one tile of tokens reads
-// (a product of at most 128 rows) is read once a step.
-__device__ __forceinline__ void tma_load_2d_stream(void* smem, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
-    unsigned long long policy;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(policy));
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;\n"
-                 ::"r"(smem_u32(smem)), "l"((unsigned long long)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(policy) : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand, rows of 128 bytes, 128-byte swizzle, groups of 8
-// rows 1024 bytes apart (the layout a TMA load with CU_TENSOR_MAP_SWIZZLE_128B writes).
-__device__ __forceinline__ unsigned long long umma_desc(unsigned smem_addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((smem_addr & 0x3FFFF) >> 4);          // start address, 16-byte units
-    d |= (unsigned long long)1 << 16;                                // leading byte offset (unused with swizzle)
-    d |= (unsigned long long)(1024 >> 4) << 32;                      // stride byte offset: 8 rows
-    d |= (unsigned long long)1 << 46;                                // descriptor version of sm_100
-    d |= (unsigned long long)2 << 61;                                // 128-byte swizzle
-    return d;
-}
-// Instruction descriptor: bfloat16 x bfloat16 -> float32, both operands K-major, M = 128, N = 256.
-__device__ __forceinline__ unsigned umma_idesc() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TC_BN >> 3) << 17) | ((unsigned)(TC_BM >> 4) << 24);
-}
-__device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b,
-                                          unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_load_32(unsigned taddr, float (&v)[32]) {
-    unsigned r[32];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 // The query/key/value projection can end in what otherwise is a kernel of its own: per-head RMSNorm of
 // queries and keys, the rotation of both by the token's position, queries to their buffer and keys and
@@ -298,7 +210,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     TcShared* sh = reinterpret_cast<TcShared*>(tiles + TC_STAGES * TC_STAGE_BYTES);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + TC_BN - 1) / TC_BN;
     const int n_tiles = tiles_m * tiles_n;
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
@@ -316,66 +228,68 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = sh->tmem_base;
+    const unsigned tmem_base = uniform(sh->tmem_base);
 
     if (warp == 0) {
-        if (lane == 0) {
+        const bool leader = elect_one();
+        if (leader) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_a) : "memory");
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_w) : "memory");
-            qil_wait_for_producer();
-            qil_release_consumer();      // the block holds its tensor memory
-            int stage = 0;
-            unsigned phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * TC_BN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&sh->empty[stage], phase ^ 1)) { atomicExch(error_word, 1); ok = false; break; }
-                    mbar_arrive_expect_tx(&sh->full[stage], TC_STAGE_BYTES);
-                    unsigned char* a_dst = tiles + stage * TC_STAGE_BYTES;
-                    tma_load_2d(a_dst, &map_a, &sh->full[stage], kb * TC_BK, m0);
-                    if (tiles_m == 1) tma_load_2d_stream(a_dst + TC_A_BYTES, &map_w, &sh->full[stage], kb * TC_BK, n0);
-                    else tma_load_2d(a_dst + TC_A_BYTES, &map_w, &sh->full[stage], kb * TC_BK, n0);
-                    if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
-                }
-            }
-            // copies still in flight land in this block's shared memory: wait for them (bounded)
-            // before the block may leave, whether or not anyone consumes them
-            for (int i = 0; i < TC_STAGES; ++i) {
-                if (!mbar_wait(&sh->empty[stage], phase ^ 1)) { atomicExch(error_word, 2); break; }
+        }
+        __syncwarp();
+        const unsigned long long policy = stream_policy();
+        qil_wait_for_producer();
+        qil_release_consumer();      // the block holds its tensor memory
+        int stage = 0;
+        unsigned phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * TC_BN;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 1); ok = false; break; }
+                mbar_arrive_expect_tx(&sh->full[stage], TC_STAGE_BYTES, leader);
+                unsigned char* a_dst = tiles + stage * TC_STAGE_BYTES;
+                tma_load_2d(a_dst, &map_a, &sh->full[stage], kb * TC_BK, m0, leader);
+                if (tiles_m == 1) tma_load_2d_stream(a_dst + TC_A_BYTES, &map_w, &sh->full[stage], kb * TC_BK, n0, policy, leader);
+                else tma_load_2d(a_dst + TC_A_BYTES, &map_w, &sh->full[stage], kb * TC_BK, n0, leader);
                 if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
             }
         }
+        // copies still in flight land in this block's shared memory: wait for them (bounded)
+        // before the block may leave, whether or not anyone consumes them
+        for (int i = 0; i < TC_STAGES; ++i) {
+            if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 2); break; }
+            if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
+        }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const unsigned idesc = umma_idesc();
-            qil_wait_for_producer();       // the bounded waits below count this kernel's own time
-            int stage = 0, acc = 0;
-            unsigned phase = 0, acc_phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                if (!mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1)) { atomicExch(error_word, 3); ok = false; break; }
+        const bool leader = elect_one();
+        const unsigned idesc = umma_idesc(TC_BM, TC_BN);
+        qil_wait_for_producer();       // the bounded waits below count this kernel's own time
+        int stage = 0, acc = 0;
+        unsigned phase = 0, acc_phase = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            if (!warp_mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1)) { if (leader) atomicExch(error_word, 3); ok = false; break; }
+            tc_fence_after();
+            const unsigned tmem_d = tmem_base + (unsigned)acc * TC_BN;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!warp_mbar_wait(&sh->full[stage], phase)) { if (leader) atomicExch(error_word, 4); ok = false; break; }
                 tc_fence_after();
-                const unsigned tmem_d = tmem_base + (unsigned)acc * TC_BN;
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&sh->full[stage], phase)) { atomicExch(error_word, 4); ok = false; break; }
-                    tc_fence_after();
-                    const unsigned a_addr = smem_u32(tiles + stage * TC_STAGE_BYTES);
-                    const unsigned b_addr = a_addr + TC_A_BYTES;
+                const unsigned a_addr = smem_u32(tiles + stage * TC_STAGE_BYTES);
+                const unsigned b_addr = a_addr + TC_A_BYTES;
 #pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k) {
-                        // 16 k-values are 32 bytes: advance the start address inside the swizzled row
-                        umma_bf16(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc,
-                                  (kb | k) ? 1u : 0u);
-                    }
-                    umma_commit(&sh->empty[stage]);      // the stage is free once these MMAs have read it
-                    if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
+                for (int k = 0; k < TC_BK / 16; ++k) {
+                    // 16 k-values are 32 bytes: advance the start address inside the swizzled row
+                    umma_bf16(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc,
+                              (kb | k) ? 1u : 0u, leader);
                 }
-                if (!ok) break;
-                umma_commit(&sh->acc_full[acc]);          // the accumulator is complete once all MMAs are done
-                acc ^= 1;
-                if (acc == 0) acc_phase ^= 1;
+                umma_commit(&sh->empty[stage], leader);      // the stage is free once these MMAs have read it
+                if (++stage == TC_STAGES) { stage = 0; phase ^= 1; }
             }
+            if (!ok) break;
+            umma_commit(&sh->acc_full[acc], leader);          // the accumulator is complete once all MMAs are done
+            acc ^= 1;
+            if (acc == 0) acc_phase ^= 1;
         }
     } else {
         const int quarter = warp & 3;                      // the TMEM lanes this warp may read
@@ -444,29 +358,27 @@ __device__ __forceinline__ void mbar_arrive_cluster(unsigned cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }
 // A tile copy of a block of a pair; `bar_cluster` may be a barrier of the pair's other block.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* map, unsigned bar_cluster, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
-                 ::"r"(smem_u32(smem)), "l"((unsigned long long)map), "r"(bar_cluster), "r"(x), "r"(y) : "memory");
+__device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* map, unsigned bar_cluster, int x, int y, bool leader) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+                 "@p cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}\n"
+                 ::"r"(smem_u32(smem)), "l"((unsigned long long)map), "r"(bar_cluster), "r"(x), "r"(y), "r"((unsigned)leader) : "memory");
 }
 __device__ __forceinline__ void umma_bf16_pair(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b,
-                                               unsigned idesc, unsigned accumulate) {
+                                               unsigned idesc, unsigned accumulate, bool leader) {
     const unsigned zero = 0u;
-    asm volatile("{\n\t.reg .pred p;\n\t"
+    asm volatile("{\n\t.reg .pred p, q;\n\t"
                  "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}\n"
-                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero) : "memory");
+                 "setp.ne.b32 q, %6, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}\n"
+                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero), "r"((unsigned)leader) : "memory");
 }
 // Arrives, once the pair's MMAs so far are done, on the barrier at this offset in both blocks.
-__device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
+__device__ __forceinline__ void umma_commit_pair(unsigned long long* bar, bool leader) {
     const unsigned short both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-                 ::"r"(smem_u32(bar)), "h"(both) : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
+                 "@p tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}\n"
+                 ::"r"(smem_u32(bar)), "h"(both), "r"((unsigned)leader) : "memory");
 }
-// bfloat16 x bfloat16 -> float32, both operands K-major, M = 256 over the pair, N = 256.
-__device__ __forceinline__ unsigned umma_idesc_pair() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(256 >> 3) << 17) | ((unsigned)(256 >> 4) << 24);
-}
-
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const bf16* __restrict__ bias, const bf16* residual, bf16* out,
@@ -474,7 +386,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     Tc2Shared* sh = reinterpret_cast<Tc2Shared*>(tiles + T2_STAGES * T2_STAGE_BYTES);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank();
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int tiles_m = (M + 255) / 256, tiles_n = (N + TC_BN - 1) / TC_BN;
@@ -495,59 +407,62 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncthreads();
     cluster_sync_all();          // the other block's barriers are initialised before anything arrives on them
     tc_fence_after();
-    const unsigned tmem_base = sh->tmem_base;
+    const unsigned tmem_base = uniform(sh->tmem_base);
 
     if (warp == 0) {
-        if (lane == 0) {
+        const bool leader = elect_one();
+        if (leader) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_a) : "memory");
             asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_w) : "memory");
-            qil_wait_for_producer();
-            qil_release_consumer();      // the block holds its tensor memory
-            int stage = 0;
-            unsigned phase = 0;
-            bool ok = true;
-            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                const int m0 = (tile % tiles_m) * 256 + (int)rank * 128, n0 = (tile / tiles_m) * TC_BN + (int)rank * 128;
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&sh->empty[stage], phase ^ 1)) { atomicExch(error_word, 1); ok = false; break; }
-                    if (rank == 0) mbar_arrive_expect_tx(&sh->full[stage], 2 * T2_STAGE_BYTES);
-                    const unsigned full_of_first = map_to_rank(smem_u32(&sh->full[stage]), 0);
-                    unsigned char* a_dst = tiles + stage * T2_STAGE_BYTES;
-                    tma_load_2d_pair(a_dst, &map_a, full_of_first, kb * TC_BK, m0);
-                    tma_load_2d_pair(a_dst + T2_A_BYTES, &map_w, full_of_first, kb * TC_BK, n0);
-                    if (++stage == T2_STAGES) { stage = 0; phase ^= 1; }
-                }
-            }
-            for (int i = 0; i < T2_STAGES; ++i) {      // this block's copies in flight land before it leaves
-                if (!mbar_wait(&sh->empty[stage], phase ^ 1)) { atomicExch(error_word, 2); break; }
+        }
+        __syncwarp();
+        const unsigned full_of_first = uniform(map_to_rank(smem_u32(sh->full), 0));
+        qil_wait_for_producer();
+        qil_release_consumer();      // the block holds its tensor memory
+        int stage = 0;
+        unsigned phase = 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int m0 = (tile % tiles_m) * 256 + (int)rank * 128, n0 = (tile / tiles_m) * TC_BN + (int)rank * 128;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 1); ok = false; break; }
+                mbar_arrive_expect_tx(&sh->full[stage], 2 * T2_STAGE_BYTES, leader && rank == 0);
+                unsigned char* a_dst = tiles + stage * T2_STAGE_BYTES;
+                tma_load_2d_pair(a_dst, &map_a, full_of_first + stage * 8, kb * TC_BK, m0, leader);
+                tma_load_2d_pair(a_dst + T2_A_BYTES, &map_w, full_of_first + stage * 8, kb * TC_BK, n0, leader);
                 if (++stage == T2_STAGES) { stage = 0; phase ^= 1; }
             }
         }
+        for (int i = 0; i < T2_STAGES; ++i) {      // this block's copies in flight land before it leaves
+            if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 2); break; }
+            if (++stage == T2_STAGES) { stage = 0; phase ^= 1; }
+        }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            const unsigned idesc = umma_idesc_pair();
+        if (rank == 0) {
+            const bool leader = elect_one();
+            const unsigned idesc = umma_idesc(256, TC_BN);
             qil_wait_for_producer();
             int stage = 0, acc = 0;
             unsigned phase = 0, acc_phase = 0;
             bool ok = true;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                if (!mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1)) { atomicExch(error_word, 3); ok = false; break; }
+                if (!warp_mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1)) { if (leader) atomicExch(error_word, 3); ok = false; break; }
                 tc_fence_after();
                 const unsigned tmem_d = tmem_base + (unsigned)acc * TC_BN;
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&sh->full[stage], phase)) { atomicExch(error_word, 4); ok = false; break; }
+                    if (!warp_mbar_wait(&sh->full[stage], phase)) { if (leader) atomicExch(error_word, 4); ok = false; break; }
                     tc_fence_after();
                     const unsigned a_addr = smem_u32(tiles + stage * T2_STAGE_BYTES);
                     const unsigned b_addr = a_addr + T2_A_BYTES;
 #pragma unroll
                     for (int k = 0; k < TC_BK / 16; ++k)
                         umma_bf16_pair(tmem_d, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc,
-                                       (kb | k) ? 1u : 0u);
-                    umma_commit_pair(&sh->empty[stage]);
+                                       (kb | k) ? 1u : 0u, leader);
+                    umma_commit_pair(&sh->empty[stage], leader);
                     if (++stage == T2_STAGES) { stage = 0; phase ^= 1; }
                 }
                 if (!ok) break;
-                umma_commit_pair(&sh->acc_full[acc]);
+                umma_commit_pair(&sh->acc_full[acc], leader);
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }
@@ -636,7 +551,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     TrShared* sh = reinterpret_cast<TrShared*>(ring + Shape::STAGES * Shape::STAGE_BYTES);
     float* sums = reinterpret_cast<float*>(ring);          // [ROWS][128] once the ring is read out
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank(), blocks = cluster_blocks();
     const int n0 = blockIdx.x / blocks * TR_BM;
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
@@ -655,55 +570,54 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = sh->tmem_base;
+    const unsigned tmem_base = uniform(sh->tmem_base);
 
     if (warp == 0) {
-        if (lane == 0) {
-            // the ring's first round: weights, which no kernel writes, before the kernel before this one has ended
-            const int first = kb1 - kb0 < Shape::STAGES ? kb1 - kb0 : Shape::STAGES;
-            for (int s = 0; s < first; ++s) {
-                mbar_arrive_expect_tx(&sh->full[s], Shape::STAGE_BYTES);
-                tma_load_2d_stream(ring + s * Shape::STAGE_BYTES, &map_w, &sh->full[s], (kb0 + s) * TC_BK, n0);
-            }
-            qil_wait_for_producer();
-            qil_release_consumer();
-            for (int s = 0; s < first; ++s)
-                tma_load_2d(ring + s * Shape::STAGE_BYTES + TR_W_BYTES, &map_x, &sh->full[s], (kb0 + s) * TC_BK, 0);
-            int stage = first == Shape::STAGES ? 0 : first;
-            unsigned phase = first == Shape::STAGES ? 1 : 0;
-            for (int kb = kb0 + first; kb < kb1; ++kb) {
-                if (!mbar_wait(&sh->empty[stage], phase ^ 1)) { atomicExch(error_word, 1); break; }
-                mbar_arrive_expect_tx(&sh->full[stage], Shape::STAGE_BYTES);
-                unsigned char* to = ring + stage * Shape::STAGE_BYTES;
-                tma_load_2d_stream(to, &map_w, &sh->full[stage], kb * TC_BK, n0);
-                tma_load_2d(to + TR_W_BYTES, &map_x, &sh->full[stage], kb * TC_BK, 0);
-                if (++stage == Shape::STAGES) { stage = 0; phase ^= 1; }
-            }
-            for (int i = 0; i < first; ++i) {      // copies in flight land before the block may leave
-                const int back = (stage + Shape::STAGES - first + i) % Shape::STAGES;
-                const unsigned round = (unsigned)((kb1 - kb0 - first + i) / Shape::STAGES) & 1;
-                if (!mbar_wait(&sh->empty[back], round)) { atomicExch(error_word, 2); break; }
-            }
+        const bool leader = elect_one();
+        const unsigned long long policy = stream_policy();
+        // the ring's first round: weights, which no kernel writes, before the kernel before this one has ended
+        const int first = kb1 - kb0 < Shape::STAGES ? kb1 - kb0 : Shape::STAGES;
+        for (int s = 0; s < first; ++s) {
+            mbar_arrive_expect_tx(&sh->full[s], Shape::STAGE_BYTES, leader);
+            tma_load_2d_stream(ring + s * Shape::STAGE_BYTES, &map_w, &sh->full[s], (kb0 + s) * TC_BK, n0, policy, leader);
+        }
+        qil_wait_for_producer();
+        qil_release_consumer();
+        for (int s = 0; s < first; ++s)
+            tma_load_2d(ring + s * Shape::STAGE_BYTES + TR_W_BYTES, &map_x, &sh->full[s], (kb0 + s) * TC_BK, 0, leader);
+        int stage = first == Shape::STAGES ? 0 : first;
+        unsigned phase = first == Shape::STAGES ? 1 : 0;
+        for (int kb = kb0 + first; kb < kb1; ++kb) {
+            if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 1); break; }
+            mbar_arrive_expect_tx(&sh->full[stage], Shape::STAGE_BYTES, leader);
+            unsigned char* to = ring + stage * Shape::STAGE_BYTES;
+            tma_load_2d_stream(to, &map_w, &sh->full[stage], kb * TC_BK, n0, policy, leader);
+            tma_load_2d(to + TR_W_BYTES, &map_x, &sh->full[stage], kb * TC_BK, 0, leader);
+            if (++stage == Shape::STAGES) { stage = 0; phase ^= 1; }
+        }
+        for (int i = 0; i < first; ++i) {      // copies in flight land before the block may leave
+            const int back = (stage + Shape::STAGES - first + i) % Shape::STAGES;
+            const unsigned round = (unsigned)((kb1 - kb0 - first + i) / Shape::STAGES) & 1;
+            if (!warp_mbar_wait(&sh->empty[back], round)) { if (leader) atomicExch(error_word, 2); break; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(ROWS >> 3) << 17) | ((unsigned)(TR_BM >> 4) << 24);
-            qil_wait_for_producer();       // the rows come after it; the bounded waits count this kernel's own time
-            int stage = 0;
-            unsigned phase = 0;
-            bool ok = true;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(&sh->full[stage], phase)) { atomicExch(error_word, 4); ok = false; break; }
-                tc_fence_after();
-                const unsigned w_addr = smem_u32(ring + stage * Shape::STAGE_BYTES), x_addr = w_addr + TR_W_BYTES;
+        const bool leader = elect_one();
+        const unsigned idesc = umma_idesc(TR_BM, ROWS);
+        qil_wait_for_producer();       // the rows come after it; the bounded waits count this kernel's own time
+        int stage = 0;
+        unsigned phase = 0;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            if (!warp_mbar_wait(&sh->full[stage], phase)) { if (leader) atomicExch(error_word, 4); ok = false; break; }
+            tc_fence_after();
+            const unsigned w_addr = smem_u32(ring + stage * Shape::STAGE_BYTES), x_addr = w_addr + TR_W_BYTES;
 #pragma unroll
-                for (int k = 0; k < TC_BK / 16; ++k)
-                    umma_bf16(tmem_base, umma_desc(w_addr + k * 32), umma_desc(x_addr + k * 32), idesc, (kb > kb0 || k) ? 1u : 0u);
-                umma_commit(&sh->empty[stage]);
-                if (++stage == Shape::STAGES) { stage = 0; phase ^= 1; }
-            }
-            if (ok) umma_commit(&sh->acc_full);
+            for (int k = 0; k < TC_BK / 16; ++k)
+                umma_bf16(tmem_base, umma_desc(w_addr + k * 32), umma_desc(x_addr + k * 32), idesc, (kb > kb0 || k) ? 1u : 0u, leader);
+            umma_commit(&sh->empty[stage], leader);
+            if (++stage == Shape::STAGES) { stage = 0; phase ^= 1; }
         }
+        if (ok) umma_commit(&sh->acc_full, leader);
     } else {
         const int quarter = warp & 3;
         qil_wait_for_producer();
