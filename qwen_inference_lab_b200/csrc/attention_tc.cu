@@ -24,8 +24,7 @@
 //
 // Every mbarrier wait is bounded (about a second), records its place in the error word when it runs
 // out and makes its role stop; the block then frees its tensor memory and returns.
-#include "common.cuh"
-#include <cuda.h>
+#include "tcgen05.cuh"
 
 QIL_ERROR_STORAGE
 
@@ -52,47 +51,10 @@ static_assert(AT_D % 16 == 0 && AT_D >= 16 && AT_D <= 128 && AT_E % 16 == 0 && A
 #define AT_VTILE (AT_ES * AT_SLAB)    // a V tile
 #define AT_TMEM_COLS (AT_N == 64 ? 256 : 512)
 #define AT_STAGES 2
-#define AT_WAIT_CYCLES 2000000000ll
 
-__device__ __forceinline__ unsigned at_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void at_mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(at_smem(bar)), "r"(count));
-}
-__device__ __forceinline__ void at_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(at_smem(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void at_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(at_smem(bar)) : "memory");
-}
-__device__ __forceinline__ bool at_try_wait(unsigned long long* bar, unsigned parity) {
-    unsigned done;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}\n"
-                 : "=r"(done) : "r"(at_smem(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ bool at_wait(unsigned long long* bar, unsigned parity) {
-    if (at_try_wait(bar, parity)) return true;
-    const long long start = clock64();
-    while (!at_try_wait(bar, parity)) {
-        if (clock64() - start > AT_WAIT_CYCLES) return false;
-    }
-    return true;
-}
 __device__ __forceinline__ void at_tma_3d(void* smem, const CUtensorMap* map, unsigned long long* bar, int x, int y, int z) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
-                 ::"r"(at_smem(smem)), "l"((unsigned long long)map), "r"(at_smem(bar)), "r"(x), "r"(y), "r"(z) : "memory");
-}
-// K-major operand: rows of 128 bytes (64 elements of k), 128-byte swizzle, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ unsigned long long at_desc_kmajor(unsigned addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((addr & 0x3FFFF) >> 4);
-    d |= (unsigned long long)1 << 16;
-    d |= (unsigned long long)(1024 >> 4) << 32;
-    d |= (unsigned long long)1 << 46;
-    d |= (unsigned long long)2 << 61;
-    return d;
+                 ::"r"(smem_u32(smem)), "l"((unsigned long long)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
 }
 // MN-major operand from the same image: 64 elements of n contiguous (one 128-byte row), rows are k;
 // the next 64 n lie one slab further (leading offset), the next 8 k lie 1024 bytes further (stride offset).
@@ -105,26 +67,16 @@ __device__ __forceinline__ unsigned long long at_desc_mnmajor(unsigned addr) {
     d |= (unsigned long long)2 << 61;
     return d;
 }
-__device__ __forceinline__ void at_mma(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned acc) {
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                 ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-}
-// The same with the first operand in tensor memory (lane = row, two 16-bit elements per 32-bit column,
+// An MMA with the first operand in tensor memory (lane = row, two 16-bit elements per 32-bit column,
 // the reduction dimension along the columns).
-__device__ __forceinline__ void at_mma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc, unsigned acc) {
+__device__ __forceinline__ void at_mma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long db, unsigned idesc, unsigned acc, bool leader) {
     const unsigned zero = 0u;
-    asm volatile("{\n\t.reg .pred p;\n\t"
+    asm volatile("{\n\t.reg .pred p, q;\n\t"
                  "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
-                 ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(zero) : "memory");
+                 "setp.ne.b32 q, %6, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(zero), "r"((unsigned)leader) : "memory");
 }
-__device__ __forceinline__ void at_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(at_smem(bar)) : "memory");
-}
-__device__ __forceinline__ void at_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void at_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
 __device__ __forceinline__ void at_tmem_ld32(unsigned taddr, unsigned (&r)[32]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -206,7 +158,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     // window is refused below rather than padded, so that two blocks fit the SM's shared memory
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = smem_raw;
-    if ((at_smem(base) & 1023u) != 0) {
+    if ((smem_u32(base) & 1023u) != 0) {
         if (threadIdx.x == 0) atomicExch(p.error_word, 31);
         return;
     }
@@ -214,7 +166,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     unsigned char* sK = sQ + AT_QTILE;                      // [stages][slabs]
     unsigned char* sV = sK + AT_STAGES * AT_KTILE;          // [stages][slabs]
     AtShared* sh = reinterpret_cast<AtShared*>(sV + AT_STAGES * AT_VTILE);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     // heads vary fastest, so all heads of the longest tile start first (tiles come sorted, longest first)
     const int head = blockIdx.x;
     const int kv_head = head / (p.n_q_heads / p.n_kv_heads);
@@ -233,26 +185,26 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     const int* table = p.block_table + (size_t)info.w * p.table_stride;
 
     if (threadIdx.x == 0) {
-        at_mbar_init(&sh->q_full, 1);
+        mbar_init(&sh->q_full, 1);
         for (int s = 0; s < AT_STAGES; ++s) {
-            at_mbar_init(&sh->k_full[s], 1); at_mbar_init(&sh->k_empty[s], 1);
-            at_mbar_init(&sh->v_full[s], 1); at_mbar_init(&sh->v_empty[s], 1);
+            mbar_init(&sh->k_full[s], 1); mbar_init(&sh->k_empty[s], 1);
+            mbar_init(&sh->v_full[s], 1); mbar_init(&sh->v_empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b) at_mbar_init(&sh->s_full[b], 1);
-        at_mbar_init(&sh->p_full[0], 4);
-        at_mbar_init(&sh->p_full[1], 4);
-        at_mbar_init(&sh->pv_done, 1);
+        for (int b = 0; b < 2; ++b) mbar_init(&sh->s_full[b], 1);
+        mbar_init(&sh->p_full[0], 4);
+        mbar_init(&sh->p_full[1], 4);
+        mbar_init(&sh->pv_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
-                     ::"r"(at_smem(&sh->tmem_base)), "r"((unsigned)AT_TMEM_COLS) : "memory");
+                     ::"r"(smem_u32(&sh->tmem_base)), "r"((unsigned)AT_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    at_fence_before();
+    tc_fence_before();
     __syncthreads();
-    at_fence_after();
-    const unsigned tmem = sh->tmem_base;
+    tc_fence_after();
+    const unsigned tmem = uniform(sh->tmem_base);
     auto tmem_s = [tmem](int buffer) { return tmem + (unsigned)(buffer * AT_N); };    // the two score buffers
     const unsigned tmem_o = tmem + 2u * AT_N;
 
@@ -271,7 +223,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (kv == 0) {
                 asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_q) : "memory");
                 // queries: box (64 elements, 1 head, 128 tokens) per slab of the head
-                at_expect_tx(&sh->q_full, AT_QTILE);
+                mbar_arrive_expect_tx(&sh->q_full, AT_QTILE, true);
                 for (int slab = 0; slab < AT_DS; ++slab) at_tma_3d(sQ + slab * AT_QSLAB, &map_q, &sh->q_full, slab * 64, head, n0);
             }
         }
@@ -298,11 +250,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             const int pg = lane % pages_per_tile, slab = (lane / pages_per_tile) & 1;
             const int page = __shfl_sync(0xffffffffu, my_page, (j % tiles_per_batch) * pages_per_tile + pg);
             if (lane == 0) {
-                if (!at_wait(&empty[stage], parity)) {
+                if (!mbar_wait(&empty[stage], parity)) {
                     atomicExch(p.error_word, 11);
                     ok = 0;
                 } else {
-                    at_expect_tx(&full[stage], (unsigned)(pages * slabs * page_bytes));
+                    mbar_arrive_expect_tx(&full[stage], (unsigned)(pages * slabs * page_bytes), true);
                 }
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -315,60 +267,59 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         // leave only after the copies have been consumed or have had a second to land
         if (lane == 0 && ok) {
             for (int j = n_tiles; j < n_tiles + AT_STAGES; ++j) {
-                if (!at_wait(&empty[j % AT_STAGES], ((j / AT_STAGES) & 1) ^ 1)) {
+                if (!mbar_wait(&empty[j % AT_STAGES], ((j / AT_STAGES) & 1) ^ 1)) {
                     atomicExch(p.error_word, 12);
                     break;
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // bfloat16 -> float32, M = 128; scores: N = keys; output: N = the value slabs' columns, B (V) read MN-major
-            const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(AT_N >> 3) << 17) | ((unsigned)(AT_M >> 4) << 24);
-            const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(AT_ES * 64 >> 3) << 17) | ((unsigned)(AT_M >> 4) << 24);
-            bool ok = at_wait(&sh->q_full, 0);
-            if (!ok) atomicExch(p.error_word, 13);
-            auto issue_scores = [&](int j) -> bool {
-                const int stage = j % AT_STAGES, buf = j & 1;
-                if (!at_wait(&sh->k_full[stage], (j / AT_STAGES) & 1)) { atomicExch(p.error_word, 14); return false; }
-                // The score buffer of tile j held P of tile j - 2: the MMA that read it was issued before this one
-                // and MMAs run in the order of their issue, so the buffer needs no barrier of its own.
-                at_fence_after();
-                const unsigned q_addr = at_smem(sQ), k_addr = at_smem(sK + stage * AT_KTILE);
+        // bfloat16 -> float32, M = 128; scores: N = keys; output: N = the value slabs' columns, B (V) read MN-major
+        const bool leader = elect_one();
+        const unsigned idesc_s = umma_idesc(AT_M, AT_N);
+        const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(AT_ES * 64 >> 3) << 17) | ((unsigned)(AT_M >> 4) << 24);
+        bool ok = warp_mbar_wait(&sh->q_full, 0);
+        if (!ok && leader) atomicExch(p.error_word, 13);
+        auto issue_scores = [&](int j) -> bool {
+            const int stage = j % AT_STAGES, buf = j & 1;
+            if (!warp_mbar_wait(&sh->k_full[stage], (j / AT_STAGES) & 1)) { if (leader) atomicExch(p.error_word, 14); return false; }
+            // The score buffer of tile j held P of tile j - 2: the MMA that read it was issued before this one
+            // and MMAs run in the order of their issue, so the buffer needs no barrier of its own.
+            tc_fence_after();
+            const unsigned q_addr = smem_u32(sQ), k_addr = smem_u32(sK + stage * AT_KTILE);
 #pragma unroll
-                for (int kk = 0; kk < AT_D / 16; ++kk) {
-                    // slab of the head, then 16 elements = 32 bytes inside the 128-byte row
-                    at_mma(tmem_s(buf), at_desc_kmajor(q_addr + (kk >> 2) * AT_QSLAB + (kk & 3) * 32),
-                           at_desc_kmajor(k_addr + (kk >> 2) * AT_SLAB + (kk & 3) * 32), idesc_s, kk ? 1u : 0u);
-                }
-                at_commit(&sh->s_full[buf]);
-                at_commit(&sh->k_empty[stage]);
-                AT_STAMP(1, 4 * j);
-                return true;
-            };
-            if (ok) ok = issue_scores(0);
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                if (j + 1 < n_tiles) { ok = issue_scores(j + 1); if (!ok) break; }
-                const int stage = j % AT_STAGES;
-                if (!at_wait(&sh->v_full[stage], (j / AT_STAGES) & 1)) { atomicExch(p.error_word, 16); ok = false; break; }
-                AT_STAMP(1, 4 * j + 1);
-                // one barrier per score buffer: the softmax may publish P of the next tile before this thread has
-                // looked at this tile's barrier (nothing holds it back but the scores, which are issued above),
-                // and a single barrier would then be two phases on, which a parity cannot tell from none
-                if (!at_wait(&sh->p_full[j & 1], (j >> 1) & 1)) { atomicExch(p.error_word, 17); ok = false; break; }
-                AT_STAMP(1, 4 * j + 2);
-                at_fence_after();
-                const unsigned v_addr = at_smem(sV + stage * AT_VTILE);
-#pragma unroll
-                for (int kk = 0; kk < AT_N / 16; ++kk) {
-                    // P: 16 keys = 8 columns of tensor memory; V: 16 keys = 16 rows of 128 bytes
-                    at_mma_ts(tmem_o, tmem_s(j & 1) + kk * 8, at_desc_mnmajor(v_addr + kk * 2048), idesc_pv,
-                              (j | kk) ? 1u : 0u);
-                }
-                at_commit(&sh->pv_done);
-                at_commit(&sh->v_empty[stage]);
-                AT_STAMP(1, 4 * j + 3);
+            for (int kk = 0; kk < AT_D / 16; ++kk) {
+                // slab of the head, then 16 elements = 32 bytes inside the 128-byte row
+                umma_bf16(tmem_s(buf), umma_desc(q_addr + (kk >> 2) * AT_QSLAB + (kk & 3) * 32),
+                       umma_desc(k_addr + (kk >> 2) * AT_SLAB + (kk & 3) * 32), idesc_s, kk ? 1u : 0u, leader);
             }
+            umma_commit(&sh->s_full[buf], leader);
+            umma_commit(&sh->k_empty[stage], leader);
+            if (leader) AT_STAMP(1, 4 * j);
+            return true;
+        };
+        if (ok) ok = issue_scores(0);
+        for (int j = 0; j < n_tiles && ok; ++j) {
+            if (j + 1 < n_tiles) { ok = issue_scores(j + 1); if (!ok) break; }
+            const int stage = j % AT_STAGES;
+            if (!warp_mbar_wait(&sh->v_full[stage], (j / AT_STAGES) & 1)) { if (leader) atomicExch(p.error_word, 16); ok = false; break; }
+            if (leader) AT_STAMP(1, 4 * j + 1);
+            // one barrier per score buffer: the softmax may publish P of the next tile before this thread has
+            // looked at this tile's barrier (nothing holds it back but the scores, which are issued above),
+            // and a single barrier would then be two phases on, which a parity cannot tell from none
+            if (!warp_mbar_wait(&sh->p_full[j & 1], (j >> 1) & 1)) { if (leader) atomicExch(p.error_word, 17); ok = false; break; }
+            if (leader) AT_STAMP(1, 4 * j + 2);
+            tc_fence_after();
+            const unsigned v_addr = smem_u32(sV + stage * AT_VTILE);
+#pragma unroll
+            for (int kk = 0; kk < AT_N / 16; ++kk) {
+                // P: 16 keys = 8 columns of tensor memory; V: 16 keys = 16 rows of 128 bytes
+                at_mma_ts(tmem_o, tmem_s(j & 1) + kk * 8, at_desc_mnmajor(v_addr + kk * 2048), idesc_pv,
+                          (j | kk) ? 1u : 0u, leader);
+            }
+            umma_commit(&sh->pv_done, leader);
+            umma_commit(&sh->v_empty[stage], leader);
+            if (leader) AT_STAMP(1, 4 * j + 3);
         }
     } else if (warp < AT_VALUE_WARP) {
         const int quarter = warp & 3;
@@ -390,9 +341,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int buf = j & 1, stage = j % AT_STAGES;
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j);
-            if (!at_wait(&sh->s_full[buf], (j >> 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 21); ok = false; break; }
+            if (!mbar_wait(&sh->s_full[buf], (j >> 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 21); ok = false; break; }
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j + 1);
-            at_fence_after();
+            tc_fence_after();
             float s[AT_N];
             {
                 unsigned r[AT_N / 32][32];
@@ -471,8 +422,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 // second MMA waits for this warp.  After it, it could also be a phase behind (another warp still at its
                 // rescale of the tile before), which the parity of the last wait below cannot tell from done: so the
                 // last tile waits here whether it rescales or not.  Its second MMA follows the awaited one anyway.
-                if (!at_wait(&sh->pv_done, (j - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 22); ok = false; break; }
-                at_fence_after();
+                if (!mbar_wait(&sh->pv_done, (j - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 22); ok = false; break; }
+                tc_fence_after();
             }
             if (rescale) {
 #pragma unroll 1
@@ -490,7 +441,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             // on the last tile, value rows past the last visible key may hold anything (unwritten slots):
             // zero them so that 0 * garbage cannot become NaN; they are this thread's key row
             if (j == n_tiles - 1) {
-                if (!at_wait(&sh->v_full[stage], (j / AT_STAGES) & 1)) { if (lane == 0) atomicExch(p.error_word, 23); ok = false; break; }
+                if (!mbar_wait(&sh->v_full[stage], (j / AT_STAGES) & 1)) { if (lane == 0) atomicExch(p.error_word, 23); ok = false; break; }
                 if (row < AT_N && key0 + row > hi) {
                     unsigned char* v_row = sV + stage * AT_VTILE + row * 128;
 #pragma unroll
@@ -511,16 +462,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 at_wait_st();
             }
             if (j == n_tiles - 1) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // the zeroed value rows
-            at_fence_before();
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0) at_arrive(&sh->p_full[j & 1]);
+            if (lane == 0) mbar_arrive(&sh->p_full[j & 1]);
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j + 5);
         }
         if (ok) {
-            if (!at_wait(&sh->pv_done, (n_tiles - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 24); ok = false; }
+            if (!mbar_wait(&sh->pv_done, (n_tiles - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 24); ok = false; }
         }
         if (ok) {
-            at_fence_after();
+            tc_fence_after();
             if (p.sink_log2 != nullptr) l += (m_used == -INFINITY) ? 1.f : exp2f(p.sink_log2[head] - m_used);
             const float inv = l > 0.f ? 1.f / l : 0.f;
             bf16* dst = p.out + ((size_t)(n0 + row) * p.n_q_heads + head) * AT_E;
@@ -542,10 +493,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
         }
     }
-    at_fence_before();
+    tc_fence_before();
     __syncthreads();
     if (warp == 1) {
-        at_fence_after();
+        tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((unsigned)AT_TMEM_COLS) : "memory");
     }
 }
