@@ -500,6 +500,325 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
+// ------------------------------------------------------------------ two SMs on one tile, the tokens cut evenly
+// The kernel above with the operands' places changed: features lie on the accumulator's lanes (W is the MMA's A operand) and
+// tokens on its columns, because a tile may have any multiple of 16 columns.  The launch cuts the tokens into even tiles
+// (521 are three of 176 where tiles of 256 compute 768), as `tokens_a_tile` says.
+//
+// Epilogue: a lane holds a feature, memory wants a token's features side by side.  Two groups of four warps take 32 columns
+// in turn: the warps leave their lanes' float32 sums in the group's staging buffer, then take its rows (a token's 128
+// features; of the q/k/v projection a whole head), four features a lane.  Tensor memory is free for the next tile once
+// it is staged.  Barriers and bounded waits are those of the kernel above.
+#define TE_STAGES 6
+#define TE_W_BYTES (128 * TC_BK * 2)
+#define TE_STAGE_BYTES (2 * TE_W_BYTES)          // and up to 128 tokens
+#define TE_CHUNK 32                              // tokens a group stages at a time
+#define TE_STAGING_BYTES (TE_CHUNK * 128 * 4)
+
+struct TcEvenShared {
+    unsigned long long full[TE_STAGES];
+    unsigned long long empty[TE_STAGES];
+    unsigned long long acc_full[2];
+    unsigned long long acc_empty[2];
+    unsigned tmem_base;
+    unsigned pad;
+};
+
+// One token's head of the q/k/v projection, four values a lane (`f`: the product, with its bias): the arithmetic and the
+// rounding points of tc_store_qkv_head, the sum of squares as a tree over the lanes.  cf, sf: the lane's cosines and sines.
+__device__ __forceinline__ uint2 te_qkv_values(const float4& f, const bf16* norm_w, bool rotate, const float4& cf, const float4& sf,
+                                               float eps, int lane) {
+    typedef __nv_bfloat162 bf2;
+    bf2 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
+    if (norm_w != nullptr) {
+        const float2 a = __bfloat1622float2(lo), b = __bfloat1622float2(hi);
+        const float sq = warp_sum(fmaf(b.y, b.y, fmaf(b.x, b.x, fmaf(a.y, a.y, a.x * a.x))));
+        const float scale = rsqrtf(sq / 128.0f + eps);
+        const uint2 w = *reinterpret_cast<const uint2*>(norm_w + lane * 4);
+        lo = __hmul2_rn(__floats2bfloat162_rn(a.x * scale, a.y * scale), *reinterpret_cast<const bf2*>(&w.x));
+        hi = __hmul2_rn(__floats2bfloat162_rn(b.x * scale, b.y * scale), *reinterpret_cast<const bf2*>(&w.y));
+    }
+    if (rotate) {
+        // the table holds values already rounded to bfloat16: the conversion is exact
+        const bf2 c0 = __floats2bfloat162_rn(cf.x, cf.y), c1 = __floats2bfloat162_rn(cf.z, cf.w);
+        const bf2 s0 = __floats2bfloat162_rn(sf.x, sf.y), s1 = __floats2bfloat162_rn(sf.z, sf.w);
+        // lanes 0..15 hold the first half of the head, lane + 16 the partners of a lane's values
+        const unsigned other_lo = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<const unsigned*>(&lo), 16);
+        const unsigned other_hi = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<const unsigned*>(&hi), 16);
+        const bf2 p0 = *reinterpret_cast<const bf2*>(&other_lo), p1 = *reinterpret_cast<const bf2*>(&other_hi);
+        // every product and sum rounds by itself (the _rn forms are never contracted into fused multiply-adds)
+        if (lane < 16) {
+            lo = __hsub2_rn(__hmul2_rn(lo, c0), __hmul2_rn(p0, s0));
+            hi = __hsub2_rn(__hmul2_rn(hi, c1), __hmul2_rn(p1, s1));
+        } else {
+            lo = __hadd2_rn(__hmul2_rn(p0, s0), __hmul2_rn(lo, c0));
+            hi = __hadd2_rn(__hmul2_rn(p1, s1), __hmul2_rn(hi, c1));
+        }
+    }
+    uint2 packed;
+    packed.x = *reinterpret_cast<const unsigned*>(&lo);
+    packed.y = *reinterpret_cast<const unsigned*>(&hi);
+    return packed;
+}
+
+// The four warps of an epilogue group meet.
+__device__ __forceinline__ void te_group_sync(int group) { asm volatile("bar.sync %0, 128;\n" ::"r"(group + 1) : "memory"); }
+
+// The rows of a staged chunk that one of the group's four warps takes: tokens m0 + i of i = part, part + 4, ... < rows, the 128
+// features from n0 on.
+__device__ __forceinline__ void te_store_rows(const float* staged, int part, int rows, int m0, int n0, int N, int silu_pairs,
+                                              const bf16* __restrict__ bias, const bf16* residual, bf16* out, const TcQkvTail& tail, int lane) {
+    constexpr int R = TE_CHUNK / 4;
+    if (n0 >= N) return;
+    if (silu_pairs) {
+        // columns come as [8 gate, 8 up] groups: half a warp a token, four outputs a lane
+        const int col = ((lane & 15) >> 1) * 16 + (lane & 1) * 4;
+#pragma unroll
+        for (int r = 0; r < R; r += 2) {
+            const int i = part + 4 * (r + (lane >> 4));
+            const float4 g = *reinterpret_cast<const float4*>(staged + i * 128 + col);
+            const float4 u = *reinterpret_cast<const float4*>(staged + i * 128 + col + 8);
+            if (i >= rows || n0 + col >= N) continue;
+            const float gate[4] = {g.x, g.y, g.z, g.w}, up[4] = {u.x, u.y, u.z, u.w};
+            uint2 packed;
+            bf16* o = reinterpret_cast<bf16*>(&packed);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float x = round_to<bf16>(gate[e]);
+                const float act = round_to<bf16>(__fdividef(x, 1.0f + __expf(-x)));
+                o[e] = __float2bfloat16_rn(act * round_to<bf16>(up[e]));
+            }
+            *reinterpret_cast<uint2*>(out + (size_t)(m0 + i) * (N / 2) + n0 / 2 + (lane & 15) * 4) = packed;
+        }
+        return;
+    }
+    const int n = n0 + lane * 4;
+    const bool inside = n < N;
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bias != nullptr && inside) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(bias + n);
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        b = make_float4(x.x, x.y, y.x, y.y);
+    }
+    if (tail.q_out != nullptr) {
+        // The 128 features are one whole head, and every lane takes part in its sums.  What a row's place and rotation need is
+        // asked for once a chunk, a row a lane, and for four rows at a time: these are trips to L2, one after the other.
+        const int head = n0 / 128;
+        const bool is_q = head < tail.n_q_heads, is_k = !is_q && head < tail.n_q_heads + tail.n_kv_heads;
+        const bf16* norm_w = is_q ? tail.q_norm : (is_k ? tail.k_norm : nullptr);
+        const bool rotate = (is_q || is_k) && tail.rope != nullptr;
+        const int mine = part + 4 * (lane & (R - 1));
+        int pos_of_lane = 0, page_of_lane = -1;
+        if (mine < rows) {
+            pos_of_lane = tail.positions[m0 + mine];
+            const int index = pos_of_lane / tail.page_size;          // a position the table has no entry for writes nothing
+            if (!is_q && pos_of_lane >= 0 && index < tail.table_stride)
+                page_of_lane = tail.block_table[(size_t)tail.token_row[m0 + mine] * tail.table_stride + index];
+        }
+#pragma unroll
+        for (int r0 = 0; r0 < R; r0 += 4) {
+            float4 f[4], cf[4], sf[4];
+            int pos[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                pos[u] = __shfl_sync(0xffffffffu, pos_of_lane, r0 + u);
+                const int row = (pos[u] >= tail.rope_rows && tail.rope_rows > 0) ? tail.rope_rows - 1 : pos[u];
+                f[u] = *reinterpret_cast<const float4*>(staged + (part + 4 * (r0 + u)) * 128 + lane * 4);
+                cf[u] = sf[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (rotate && part + 4 * (r0 + u) < rows) {
+                    const float* cs = tail.rope + (size_t)row * 128 + (lane & 15) * 4;
+                    cf[u] = *reinterpret_cast<const float4*>(cs);
+                    sf[u] = *reinterpret_cast<const float4*>(cs + 64);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = part + 4 * (r0 + u), page = __shfl_sync(0xffffffffu, page_of_lane, r0 + u);
+                f[u].x += b.x; f[u].y += b.y; f[u].z += b.z; f[u].w += b.w;
+                const uint2 values = te_qkv_values(f[u], norm_w, rotate, cf[u], sf[u], tail.eps, lane);
+                if (i >= rows) continue;
+                bf16* dst;
+                if (is_q) {
+                    dst = tail.q_out + ((size_t)(m0 + i) * tail.n_q_heads + head) * 128;
+                } else {
+                    if (page < 0 || page >= tail.num_pages) continue;        // never write outside the pool
+                    const int kv_head = is_k ? head - tail.n_q_heads : head - tail.n_q_heads - tail.n_kv_heads;
+                    dst = tail.pages + ((((size_t)page * 2 + (is_k ? 0 : 1)) * tail.n_kv_heads + kv_head) * tail.page_size + pos[u] % tail.page_size) * 128;
+                }
+                *reinterpret_cast<uint2*>(dst + lane * 4) = values;
+            }
+        }
+        return;
+    }
+    if (!inside) return;
+    uint2 held[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        held[r] = make_uint2(0u, 0u);
+        if (residual != nullptr && part + 4 * r < rows) held[r] = *reinterpret_cast<const uint2*>(residual + (size_t)(m0 + part + 4 * r) * N + n);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = part + 4 * r;
+        if (i >= rows) break;
+        float4 f = *reinterpret_cast<const float4*>(staged + i * 128 + lane * 4);
+        f.x += b.x; f.y += b.y; f.z += b.z; f.w += b.w;
+        if (residual != nullptr) {
+            const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&held[r].x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&held[r].y));
+            f.x = x.x + f.x; f.y = x.y + f.y; f.z = y.x + f.z; f.w = y.y + f.w;
+        }
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
+        uint2 packed;
+        packed.x = *reinterpret_cast<const unsigned*>(&lo);
+        packed.y = *reinterpret_cast<const unsigned*>(&hi);
+        *reinterpret_cast<uint2*>(out + (size_t)(m0 + i) * N + n) = packed;
+    }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+gemm_tc_even_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                    const bf16* __restrict__ bias, const bf16* residual, bf16* out,
+                    int M, int N, int K, int nt, int silu_pairs, int* error_word, const TcQkvTail tail) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* staging = tiles + TE_STAGES * TE_STAGE_BYTES;
+    TcEvenShared* sh = reinterpret_cast<TcEvenShared*>(staging + 2 * TE_STAGING_BYTES);
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int tiles_m = (M + nt - 1) / nt, tiles_n = (N + 255) / 256;
+    const int n_tiles = tiles_m * tiles_n;
+    const int k_blocks = (K + TC_BK - 1) / TC_BK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TE_STAGES; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&sh->acc_full[a], 1); mbar_init(&sh->acc_empty[a], 2 * TC_EPILOGUE_WARPS); }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {     // the same warp of both blocks, the same address: the pair's allocation
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                     ::"r"(smem_u32(&sh->tmem_base)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // the other block's barriers are initialised before anything arrives on them
+    tc_fence_after();
+    const unsigned tmem_base = uniform(sh->tmem_base);
+
+    if (warp == 0) {
+        const bool leader = elect_one();
+        if (leader) {
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_x) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"((unsigned long long)&map_w) : "memory");
+        }
+        __syncwarp();
+        const unsigned full_of_first = uniform(map_to_rank(smem_u32(sh->full), 0));
+        const unsigned stage_bytes = 2 * (TE_W_BYTES + nt * TC_BK);            // both blocks' weights and tokens
+        // the ring's first round: weights, which no kernel writes, before the kernel before this one has ended
+        const int first = pair < n_tiles ? (k_blocks < TE_STAGES ? k_blocks : TE_STAGES) : 0;
+        const int first_n = pair / tiles_m * 256 + (int)rank * 128, first_m = pair % tiles_m * nt + (int)rank * (nt / 2);
+        for (int s = 0; s < first; ++s) {
+            mbar_arrive_expect_tx(&sh->full[s], stage_bytes, leader && rank == 0);
+            tma_load_2d_pair(tiles + s * TE_STAGE_BYTES, &map_w, full_of_first + s * 8, s * TC_BK, first_n, leader);
+        }
+        qil_wait_for_producer();
+        qil_release_consumer();      // the block holds its tensor memory
+        for (int s = 0; s < first; ++s)
+            tma_load_2d_pair(tiles + s * TE_STAGE_BYTES + TE_W_BYTES, &map_x, full_of_first + s * 8, s * TC_BK, first_m, leader);
+        int stage = first == TE_STAGES ? 0 : first;
+        unsigned phase = first == TE_STAGES ? 1 : 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int m0 = tile % tiles_m * nt + (int)rank * (nt / 2), n0 = tile / tiles_m * 256 + (int)rank * 128;
+            for (int kb = tile == pair ? first : 0; kb < k_blocks; ++kb) {
+                if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 1); ok = false; break; }
+                mbar_arrive_expect_tx(&sh->full[stage], stage_bytes, leader && rank == 0);
+                unsigned char* to = tiles + stage * TE_STAGE_BYTES;
+                tma_load_2d_pair(to, &map_w, full_of_first + stage * 8, kb * TC_BK, n0, leader);
+                tma_load_2d_pair(to + TE_W_BYTES, &map_x, full_of_first + stage * 8, kb * TC_BK, m0, leader);
+                if (++stage == TE_STAGES) { stage = 0; phase ^= 1; }
+            }
+        }
+        for (int i = 0; i < TE_STAGES; ++i) {      // this block's copies in flight land before it leaves
+            if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 2); break; }
+            if (++stage == TE_STAGES) { stage = 0; phase ^= 1; }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            const bool leader = elect_one();
+            const unsigned idesc = umma_idesc(256, nt);
+            qil_wait_for_producer();
+            int stage = 0, acc = 0;
+            unsigned phase = 0, acc_phase = 0;
+            bool ok = true;
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+                if (!warp_mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1)) { if (leader) atomicExch(error_word, 3); ok = false; break; }
+                tc_fence_after();
+                const unsigned tmem_d = tmem_base + (unsigned)acc * 256;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!warp_mbar_wait(&sh->full[stage], phase)) { if (leader) atomicExch(error_word, 4); ok = false; break; }
+                    tc_fence_after();
+                    const unsigned w_addr = smem_u32(tiles + stage * TE_STAGE_BYTES), x_addr = w_addr + TE_W_BYTES;
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; ++k)
+                        umma_bf16_pair(tmem_d, umma_desc(w_addr + k * 32), umma_desc(x_addr + k * 32), idesc, (kb | k) ? 1u : 0u, leader);
+                    umma_commit_pair(&sh->empty[stage], leader);
+                    if (++stage == TE_STAGES) { stage = 0; phase ^= 1; }
+                }
+                if (!ok) break;
+                umma_commit_pair(&sh->acc_full[acc], leader);
+                acc ^= 1;
+                if (acc == 0) acc_phase ^= 1;
+            }
+        }
+    } else {
+        const int quarter = warp & 3, group = warp < 6 ? 0 : 1;
+        float* staged = reinterpret_cast<float*>(staging + group * TE_STAGING_BYTES);
+        qil_wait_for_producer();
+        int acc = 0;
+        unsigned acc_phase = 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int m0 = (tile % tiles_m) * nt, n0 = (tile / tiles_m) * 256 + (int)rank * 128;
+            if (ok && !mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; }
+            ok = __all_sync(0xffffffffu, ok);
+            tc_fence_after();
+            const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * 256;
+            for (int c0 = group * TE_CHUNK; c0 < nt; c0 += 2 * TE_CHUNK) {
+                float v[32];
+                tmem_load_32(taddr + c0, v);
+                if (c0 + 2 * TE_CHUNK >= nt) {          // this warp's last columns: the accumulator's next tile may begin
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&sh->acc_empty[acc]), 0));
+                }
+                te_group_sync(group);                    // the rows of the chunk before have been read
+#pragma unroll
+                for (int i = 0; i < 32; ++i) staged[i * 128 + quarter * 32 + lane] = v[i];
+                te_group_sync(group);
+                const int rows = min(min(TE_CHUNK, nt - c0), M - m0 - c0);
+                te_store_rows(staged, quarter, rows, m0 + c0, n0, N, silu_pairs, bias, residual, out, tail, lane);
+                __syncwarp();
+            }
+            if (group * TE_CHUNK >= nt) {                // a tile of one chunk: nothing for the second group
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&sh->acc_empty[acc]), 0));
+            }
+            acc ^= 1;
+            if (acc == 0) acc_phase ^= 1;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // neither block leaves while the other may still read its tiles or signal it
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
 // ------------------------------------------------------------------ a few dozen rows
 // The product for the rows between a decode step's and a prompt portion's (17 to 128): its time is that of reading W
 // once, as for the decode product, but there are too many rows for mma.sync to keep up.  128 output features sit on the
@@ -748,8 +1067,74 @@ static int make_map(CUtensorMap* map, const void* base, int rows, int cols, int 
 
 extern "C" int qil_gemm_tc_min_rows() { return 17; }
 
+// How many pairs of blocks of a kernel run at a time on the current device, asked once (`known`, by device: the limit of shared memory
+// that it raises belongs to the function on a device); 0: refused.
+#define TC_MOST_DEVICES 64
+template <typename Kernel>
+static int pairs_at_a_time(Kernel kernel, int smem, int sm_count, int* known) {
+    int device = -1;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess || device < 0 || device >= TC_MOST_DEVICES) {
+        snprintf(qil_error_text, sizeof(qil_error_text), "gemm_tc: device %d is out of range", device);
+        return 0;
+    }
+    if (known[device] > 0) return known[device];
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+        snprintf(qil_error_text, sizeof(qil_error_text), "gemm_tc: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        return 0;
+    }
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(sm_count & ~1);
+    config.blockDim = dim3(TC_THREADS);
+    config.dynamicSmemBytes = smem;
+    int clusters = 0;
+    e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &config);
+    if (e != cudaSuccess || clusters <= 0) { (void)cudaGetLastError(); clusters = sm_count / 2; }
+    return known[device] = clusters < sm_count / 2 ? clusters : sm_count / 2;
+}
+
+// What a 16-wide step of K costs a tile of the even kernel, in cycles: nt / 2 of MMA, or those that bring its 128 features and
+// nt / 2 tokens to each block.  A tile of the other two costs 128.
+static int even_step(int nt) { return nt / 2 > 64 + nt / 4 ? nt / 2 : 64 + nt / 4; }
+
+// How many tokens a tile of the even kernel takes: as many as make the fewest and cheapest waves of `pairs` tiles.  `cost`: of
+// those waves, a step of K.
+static int tokens_a_tile(int M, int tiles_n, int pairs, long long* cost) {
+    int best = 256;
+    *cost = -1;
+    for (int count = (M + 255) / 256; count <= (M + 15) / 16; ++count) {
+        const int nt = ((M + count - 1) / count + 15) / 16 * 16;
+        const long long tiles = (long long)((M + nt - 1) / nt) * tiles_n, waves = (tiles + pairs - 1) / pairs;
+        if (*cost < 0 || waves * even_step(nt) < *cost) { best = nt; *cost = waves * even_step(nt); }
+        if (tiles > 8ll * pairs) break;
+    }
+    return best;
+}
+
+// Does the even kernel take the product?  Where even tiles make its waves a tenth cheaper than those of 256 (from 256
+// tokens on, pairs of blocks) or 128 tokens (one block).  Its epilogue goes through shared memory and is the slower one: a long K
+// hides it, and a single wave of tiles has it only once; that of q/k/v (`tail`) wants the long K.
+// Measured, us (the other kernels / this one, weights from memory):
+//   gate/up of 24576 x 4096: 129 tokens 60 / 48, 300 69 / 58, 521 94 / 75, 1021 137 / 136 (not taken), 2048 256 / 256 (not taken)
+//   gate/up of 6144 x 1024:  129 tokens 11.4 / 8.3, 300 12.0 / 9.9, 521 12.5 / 12.1, 1021 16.6 / 16.9 (not taken), 2048 22.6 / 26.7 (not taken)
+//   q/k/v of 6144 x 4096:    521 tokens 34.1 / 31.0, 700 34.3 / 39.7 (not taken), 1021 51.3 / 45.1, 1500 55 / 61 (not taken)
+//   q/k/v of 4096 x 1024:    521 tokens 17.5 / 17.6, 700 18.1 / 19.0, 1021 18.2 / 24.9 (none taken)
+static int even_tokens(int M, int N, int K, bool tail, int pairs, int sm_count) {
+    const int tiles_n = (N + 255) / 256;
+    long long cost;
+    const int nt = tokens_a_tile(M, tiles_n, pairs, &cost);
+    const long long tiles = (long long)((M + nt - 1) / nt) * tiles_n;
+    const long long others = M >= 256 ? (long long)((M + 255) / 256) * tiles_n : (long long)((M + TC_BM - 1) / TC_BM) * tiles_n;
+    const int at_a_time = M >= 256 ? pairs : sm_count;
+    const long long other_cost = (others + at_a_time - 1) / at_a_time * 128;
+    const bool hidden = K >= 2048 || (tiles <= pairs && !tail);
+    return hidden && 10 * cost <= 9 * other_cost ? nt : 0;
+}
+
+// nt: tokens a tile of the even kernel (0: as even_tokens says, which may be another kernel).
 static int launch_gemm_tc(const void* a, const void* w, const void* bias, const void* residual, void* out,
-                          int M, int N, int K, int silu_pairs, int sm_count, int* error_word, const TcQkvTail& tail,
+                          int M, int N, int K, int silu_pairs, int nt, int sm_count, int* error_word, const TcQkvTail& tail,
                           cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8) QIL_REFUSE("gemm_tc: K %d must be a positive multiple of 8 (16-byte rows for TMA)", K);
@@ -760,6 +1145,31 @@ static int launch_gemm_tc(const void* a, const void* w, const void* bias, const 
         QIL_REFUSE("gemm_tc: silu_pairs needs N %% 16 == 0 and neither bias nor residual");
     if (error_word == nullptr || sm_count <= 0) QIL_REFUSE("gemm_tc: needs an error word and the SM count");
     CUtensorMap map_a, map_w;
+    static int pair_env = -1;
+    if (pair_env < 0) {
+        const char* e = getenv("QIL_GEMM_TC_PAIRS");
+        pair_env = (e != nullptr && e[0] == '0') ? 0 : 1;
+    }
+    if (nt != 0 && (nt < 16 || nt > 256 || nt % 16)) QIL_REFUSE("gemm_tc: tiles of %d tokens; a multiple of 16 up to 256", nt);
+    const bool even_fits = ((uintptr_t)bias & 7) == 0;                     // its epilogue reads four values of the bias at once
+    if (nt > 0 && !even_fits) QIL_REFUSE("gemm_tc: tiles of a number of tokens want an 8-byte aligned bias");
+    static int even_known[TC_MOST_DEVICES];
+    const int smem_even = TE_STAGES * TE_STAGE_BYTES + 2 * TE_STAGING_BYTES + (int)sizeof(TcEvenShared) + 1024;
+    int even_pairs = 0;
+    if (nt > 0 || (pair_env == 1 && even_fits)) {
+        even_pairs = pairs_at_a_time(gemm_tc_even_kernel, smem_even, sm_count, even_known);
+        if (even_pairs == 0) return -1;
+        if (nt == 0) nt = even_tokens(M, N, K, tail.q_out != nullptr, even_pairs, sm_count);
+    }
+    if (nt > 0) {
+        if (make_map(&map_a, a, M, K, nt / 2)) return -1;
+        if (make_map(&map_w, w, N, K, 128)) return -1;
+        const long long tiles = (long long)((M + nt - 1) / nt) * ((N + 255) / 256);
+        if (tiles > 0x7fffffffll) QIL_REFUSE("gemm_tc: [%d, %d] x [%d, %d] is too large for one launch", M, K, N, K);
+        qil_launch_chained(gemm_tc_even_kernel, dim3(2 * (tiles < even_pairs ? (int)tiles : even_pairs)), dim3(TC_THREADS), smem_even,
+                           stream, map_a, map_w, (const bf16*)bias, (const bf16*)residual, (bf16*)out, M, N, K, nt, silu_pairs, error_word, tail);
+        QIL_CHECK_LAUNCH();
+    }
     if (make_map(&map_a, a, M, K, TC_BM)) return -1;
     if (make_map(&map_w, w, N, K, TC_BN)) return -1;
     const int smem = TC_STAGES * TC_STAGE_BYTES + (int)sizeof(TcShared) + 1024;
@@ -769,28 +1179,13 @@ static int launch_gemm_tc(const void* a, const void* w, const void* bias, const 
         if (e != cudaSuccess) QIL_REFUSE("gemm_tc: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
         configured = true;
     }
-    static int pair_env = -1;
-    if (pair_env < 0) {
-        const char* e = getenv("QIL_GEMM_TC_PAIRS");
-        pair_env = (e != nullptr && e[0] == '0') ? 0 : 1;
-    }
     if (M >= 256 && pair_env == 1) {
         // two SMs per 256 x 256 tile; the W map's box is the 128 output features one block loads
         if (make_map(&map_w, w, N, K, 128)) return -1;
         const int smem_pair = T2_STAGES * T2_STAGE_BYTES + (int)sizeof(Tc2Shared) + 1024;
-        static int pairs_resident = 0;
-        if (pairs_resident == 0) {
-            cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_pair);
-            if (e != cudaSuccess) QIL_REFUSE("gemm_tc: cannot reserve %d bytes of shared memory: %s", smem_pair, cudaGetErrorString(e));
-            cudaLaunchConfig_t config = {};
-            config.gridDim = dim3(sm_count & ~1);
-            config.blockDim = dim3(TC_THREADS);
-            config.dynamicSmemBytes = smem_pair;
-            int clusters = 0;
-            e = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel, &config);
-            if (e != cudaSuccess || clusters <= 0) { (void)cudaGetLastError(); clusters = sm_count / 2; }
-            pairs_resident = clusters < sm_count / 2 ? clusters : sm_count / 2;
-        }
+        static int pair_known[TC_MOST_DEVICES];
+        const int pairs_resident = pairs_at_a_time(gemm_tc_pair_kernel, smem_pair, sm_count, pair_known);
+        if (pairs_resident == 0) return -1;
         const int pair_tiles = ((M + 255) / 256) * ((N + TC_BN - 1) / TC_BN);
         const int pairs = pair_tiles < pairs_resident ? pair_tiles : pairs_resident;
         qil_launch_chained(gemm_tc_pair_kernel, dim3(2 * pairs), dim3(TC_THREADS), smem_pair, stream, map_a, map_w, (const bf16*)bias,
@@ -807,9 +1202,9 @@ static int launch_gemm_tc(const void* a, const void* w, const void* bias, const 
 // error_word: a device int the caller zeroes once and reads after synchronising; non-zero means a
 // bounded wait inside the kernel ran out (1-2 producer, 3-4 MMA issuer, 5 epilogue).
 extern "C" int qil_gemm_tc(const void* a, const void* w, const void* bias, const void* residual, void* out,
-                           int M, int N, int K, int silu_pairs, int sm_count, int* error_word, cudaStream_t stream) {
+                           int M, int N, int K, int silu_pairs, int nt, int sm_count, int* error_word, cudaStream_t stream) {
     TcQkvTail none = {};
-    return launch_gemm_tc(a, w, bias, residual, out, M, N, K, silu_pairs, sm_count, error_word, none, stream);
+    return launch_gemm_tc(a, w, bias, residual, out, M, N, K, silu_pairs, nt, sm_count, error_word, none, stream);
 }
 
 // The stacked query/key/value projection of heads of 128 with its tail fused (see TcQkvTail): w is
@@ -821,7 +1216,7 @@ extern "C" int qil_gemm_tc_qkv(const void* a, const void* w, const void* bias, v
                                const float* rope, int rope_rows, const void* q_norm, const void* k_norm, float eps,
                                const int* positions, const int* token_row, const int* block_table, int table_stride,
                                int n_q_heads, int n_kv_heads, int page_size, int num_pages,
-                               int M, int K, int sm_count, int* error_word, cudaStream_t stream) {
+                               int M, int K, int nt, int sm_count, int* error_word, cudaStream_t stream) {
     if (n_q_heads <= 0 || n_kv_heads < 0) QIL_REFUSE("gemm_tc_qkv: %d query heads, %d kv heads", n_q_heads, n_kv_heads);
     if (q_out == nullptr || positions == nullptr) QIL_REFUSE("gemm_tc_qkv: needs the query buffer and the positions");
     if (n_kv_heads > 0 && (pages == nullptr || token_row == nullptr || block_table == nullptr || page_size <= 0 || num_pages <= 0))
@@ -835,7 +1230,7 @@ extern "C" int qil_gemm_tc_qkv(const void* a, const void* w, const void* bias, v
     tail.table_stride = table_stride; tail.n_q_heads = n_q_heads; tail.n_kv_heads = n_kv_heads;
     tail.page_size = page_size > 0 ? page_size : 1; tail.num_pages = num_pages;
     const int N = (n_q_heads + 2 * n_kv_heads) * 128;
-    return launch_gemm_tc(a, w, bias, nullptr, q_out, M, N, K, 0, sm_count, error_word, tail, stream);
+    return launch_gemm_tc(a, w, bias, nullptr, q_out, M, N, K, 0, nt, sm_count, error_word, tail, stream);
 }
 
 // ------------------------------------------------------------------ a few dozen rows: launch

@@ -52,9 +52,10 @@ def usable(a, weight) -> bool:
             and weight.shape[1] % 8 == 0 and weight.shape[0] % 8 == 0 and a.is_contiguous())
 
 
-def gemm_tc(a, weight, bias=None, residual=None, out=None, silu_pairs=False):
+def gemm_tc(a, weight, bias=None, residual=None, out=None, silu_pairs=False, tile_tokens=0):
     """out = a @ weight.T (+ bias) (+ residual); with ``silu_pairs`` (weight rows as [8 gate, 8 up] groups)
-    out = silu(gate) * up of width N/2.  ``residual`` may be ``out``."""
+    out = silu(gate) * up of width N/2.  ``residual`` may be ``out``.  ``tile_tokens``: a multiple of 16 up to 256 has the kernel
+    with the tokens cut evenly take the product in tiles of so many; 0 leaves it to the measured rule beside the launch."""
     _need(a, "a", torch.bfloat16, 2); _need(weight, "weight", torch.bfloat16, 2)
     m, k = a.shape
     n = weight.shape[0]
@@ -75,7 +76,7 @@ def gemm_tc(a, weight, bias=None, residual=None, out=None, silu_pairs=False):
     word = error_word(a.device)
     lib = library()
     _check(lib, lib.qil_gemm_tc(_p(a), _p(weight), _p(bias), _p(residual), _p(out), c_int(m), c_int(n), c_int(k),
-                                c_int(1 if silu_pairs else 0), c_int(_sm_count), _p(word), _stream()), "gemm_tc")
+                                c_int(1 if silu_pairs else 0), c_int(tile_tokens), c_int(_sm_count), _p(word), _stream()), "gemm_tc")
     return out
 
 
@@ -131,11 +132,11 @@ def qkv_tail_usable(a, weight, head_dim, rotary_dim, norm_weights, pages) -> boo
 
 
 def gemm_tc_qkv(a, weight, bias, q_out, pages, rope_table, q_norm, k_norm, eps, positions, token_row, block_table,
-                n_q_heads, n_kv_heads, page_size):
+                n_q_heads, n_kv_heads, page_size, tile_tokens=0):
     """The stacked q/k/v projection with its tail in the epilogue: per-head RMSNorm of queries and keys,
     rotation by position, queries into ``q_out`` [M, n_q_heads * 128], keys and values into the tokens'
     pages.  ``weight`` [(n_q_heads + 2 n_kv_heads) * 128, K]; ``n_kv_heads`` 0 for a layer without
-    keys and values of its own; ``rope_table`` float32 [positions, 128] or None."""
+    keys and values of its own; ``rope_table`` float32 [positions, 128] or None.  ``tile_tokens``: see ``gemm_tc``."""
     _need(a, "a", torch.bfloat16, 2); _need(weight, "weight", torch.bfloat16, 2)
     m, k = a.shape
     if weight.shape != ((n_q_heads + 2 * n_kv_heads) * 128, k):
@@ -169,7 +170,7 @@ def gemm_tc_qkv(a, weight, bias, q_out, pages, rope_table, q_norm, k_norm, eps, 
         c_int(rope_table.shape[0] if rope_table is not None else 0), _p(q_norm), _p(k_norm), c_float(float(eps)),
         _p(positions), _p(token_row), _p(block_table), c_int(block_table.shape[1] if block_table is not None else 0),
         c_int(n_q_heads), c_int(n_kv_heads), c_int(page_size), c_int(num_pages), c_int(m), c_int(k),
-        c_int(_sm_count), _p(word), _stream()), "gemm_tc_qkv")
+        c_int(tile_tokens), c_int(_sm_count), _p(word), _stream()), "gemm_tc_qkv")
     return q_out
 
 

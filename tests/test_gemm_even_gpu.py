@@ -1,0 +1,79 @@
+"""The tcgen05 product whose tiles cut the tokens evenly: every epilogue at the edges of tiles, against 64 bits and the other kernels."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def draw(*shape, seed=0, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).bfloat16().cuda()
+
+
+@pytest.mark.parametrize("tokens", [16, 32, 48, 176, 256])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (31, 136, 64), (177, 264, 72), (521, 640, 448), (1030, 1040, 384)])
+def test_tiles_of_any_number_of_tokens(m, n, k, tokens):
+    from qwen_inference_lab_b200.kernels import gemm_tc
+    a, w, bias, residual = draw(m, k), draw(n, k, seed=1, scale=k ** -0.5), draw(n, seed=2), draw(m, n, seed=3)
+    raw = a.double() @ w.double().t()
+    wanted = raw + bias.double() + residual.double()
+    # float32 sums and one rounding to bfloat16 (half a step of 8 bits)
+    bound = 2.0 ** -8 * 1.01 * wanted.abs() + (k + 4) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + 8)
+    out = residual.clone()
+    gemm_tc.gemm_tc(a, w, bias=bias, residual=out, out=out, tile_tokens=tokens)
+    assert bool(((out.double() - wanted).abs() <= bound).all())
+    if n % 16 == 0:
+        assert torch.equal(gemm_tc.gemm_tc(a, w, silu_pairs=True, tile_tokens=tokens), silu_apart(gemm_tc, a, w, tokens))
+    gemm_tc.check()
+
+
+def silu_apart(gemm_tc, a, w, tokens):
+    from qwen_inference_lab_b200.kernels import ops
+    hidden = ops.silu_mul(gemm_tc.gemm_tc(a, w, tile_tokens=tokens), pairs8=True)
+    # the fused form divides approximately before it rounds to bfloat16
+    fused = gemm_tc.gemm_tc(a, w, silu_pairs=True, tile_tokens=tokens)
+    assert bool(((fused.double() - hidden.double()).abs() <= 2.0 ** -6 * hidden.double().abs()).all())
+    return fused
+
+
+@pytest.mark.parametrize("m,n_q,n_kv,page,bias,norms,rope", [(300, 3, 1, 8, True, True, True), (521, 4, 2, 16, False, True, True),
+                                                             (260, 2, 0, 16, False, False, False)])
+def test_the_tail_of_the_projection(m, n_q, n_kv, page, bias, norms, rope):
+    """Against the kernel with one token a lane: the sums of squares come in another order, so a normed value may round the other way."""
+    from qwen_inference_lab_b200.kernels import gemm_tc
+    from qwen_inference_lab_b200.parts.rotary import rotary_table
+    heads, k = n_q + 2 * n_kv, 256
+    a, w, b = draw(m, k), draw(heads * 128, k, seed=1, scale=0.1), draw(heads * 128, seed=2) if bias else None
+    q_norm, k_norm = ((1 + 0.3 * draw(128, seed=s)).bfloat16() if norms else None for s in (3, 4))
+    table = rotary_table(128, 10000.0, 600, torch.bfloat16).cuda() if rope else None
+    first = m // 3                             # two requests; the table has no entry for the last tokens of the second
+    positions = torch.cat([torch.arange(5, 5 + first), torch.arange(m - first)]).int().cuda()
+    token_row = torch.cat([torch.ones(first), torch.zeros(m - first)]).int().cuda()
+    per = (m - first) // page
+    block_table = torch.randperm(2 * per, generator=torch.Generator().manual_seed(5)).int().view(2, per).cuda()
+    results = []
+    for tokens in (0, 16, 96, 176, 256):
+        q = torch.full((m, n_q * 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        pages = torch.full((2 * per, 2, max(n_kv, 1), page, 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        gemm_tc.gemm_tc_qkv(a, w, b, q, pages if n_kv else None, table, q_norm, k_norm, 1e-5, positions, token_row, block_table, n_q, n_kv,
+                            page, tile_tokens=tokens)
+        gemm_tc.check()
+        results.append((q, pages))
+    for q, pages in results[1:]:
+        for got, wanted in ((q, results[0][0]), (pages, results[0][1])):
+            assert torch.equal(got == 7.0, wanted == 7.0) or not norms
+            difference = (got.double() - wanted.double()).abs()
+            assert float((difference > 0).double().mean()) < 0.02
+            # one step of bfloat16 in the normed value, and the rotation's three roundings on top, of values up to the row's largest
+            assert float(difference.max()) <= 4 * 2.0 ** -7 * float(wanted.double().abs().max())
+
+
+def test_the_rule_takes_ragged_portions_and_leaves_whole_ones(monkeypatch):
+    """The same product with and without the rule: the kernels agree to the last rounding."""
+    from qwen_inference_lab_b200.kernels import gemm_tc
+    w = draw(2048, 2048, scale=2048 ** -0.5)
+    for m in (129, 255, 256, 257, 300, 512, 521):
+        a = draw(m, 2048, seed=m)
+        wanted = a.double() @ w.double().t()
+        got = gemm_tc.gemm_tc(a, w)
+        assert bool(((got.double() - wanted).abs() <= 2.0 ** -8 * 1.01 * wanted.abs() + 2100 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())).all())
+    gemm_tc.check()
