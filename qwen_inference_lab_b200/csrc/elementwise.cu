@@ -103,6 +103,7 @@ rmsnorm_bf16x8_kernel(const bf16* __restrict__ x, const W* __restrict__ weight, 
     __shared__ float scratch[8];
     qil_wait_for_producer();
     qil_release_consumer();
+    static_assert(RMS_VPT == 4 && (TPR == 32 || TPR == 256), "the sum's order below");
     const int tid = threadIdx.x % TPR, r = blockIdx.x * (blockDim.x / TPR) + threadIdx.x / TPR;
     const bool live = r < n_rows;                 // uniform over a row's threads
     const int src_row = !live ? 0 : rows ? rows[r] : r;
@@ -115,23 +116,29 @@ rmsnorm_bf16x8_kernel(const bf16* __restrict__ x, const W* __restrict__ weight, 
         const int idx = tid + i * TPR;
         v[i] = idx < vectors ? src[idx] : make_uint4(0u, 0u, 0u, 0u);
     }
-    float sq = 0.f;
+    // The sum of the squares has one order whatever TPR is, that of 256 threads a row: a thread its vectors' one after the
+    // other, lanes as a tree, then the eight warps as a tree.  A warp on its own keeps the first four of those warps apart
+    // (of a row of up to 1024 the other four have nothing).
+    float sq[RMS_VPT] = {};
 #pragma unroll
     for (int i = 0; i < RMS_VPT; ++i) {
         const bf16* e = reinterpret_cast<const bf16*>(&v[i]);
+        float& into = sq[TPR == 32 ? i : 0];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) { const float f = __bfloat162float(e[k]); sq += f * f; }
+        for (int k = 0; k < 8; ++k) { const float f = __bfloat162float(e[k]); into += f * f; }
     }
-    sq = warp_sum(sq);
-    if (TPR > 32) {                               // the row's warps, in their order
-        const int warp = threadIdx.x >> 5, first = warp / (TPR / 32) * (TPR / 32);
-        if ((threadIdx.x & 31) == 0) scratch[warp] = sq;
+    float total;
+    if (TPR == 32) {
+#pragma unroll
+        for (int i = 0; i < RMS_VPT; ++i) sq[i] = warp_sum(sq[i]);
+        total = (sq[0] + sq[2]) + (sq[1] + sq[3]);
+    } else {
+        sq[0] = warp_sum(sq[0]);
+        if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = sq[0];
         __syncthreads();
-        sq = scratch[first];
-#pragma unroll
-        for (int i = 1; i < TPR / 32; ++i) sq += scratch[first + i];
+        total = ((scratch[0] + scratch[4]) + (scratch[2] + scratch[6])) + ((scratch[1] + scratch[5]) + (scratch[3] + scratch[7]));
     }
-    const float scale = 1.0f / sqrtf(sq / (float)width + eps);
+    const float scale = 1.0f / sqrtf(total / (float)width + eps);
 #pragma unroll
     for (int i = 0; i < RMS_VPT; ++i) {
         const int idx = tid + i * TPR;

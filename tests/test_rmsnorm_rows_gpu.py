@@ -21,3 +21,38 @@ def test_rmsnorm_of_many_and_few_rows(width, weight_dtype):
         assert torch.equal(ops.rmsnorm(x[:n], w, 1e-6), whole[:n]), n           # a row is the same bits in any company
     rows = torch.tensor([600, 0, 7], dtype=torch.int32).cuda()
     assert torch.equal(ops.rmsnorm(x, w, 1e-6, rows=rows), whole[rows.long()])
+
+
+def in_the_order_of_256_threads(x, w, eps):
+    """The norm in float32 on the CPU: thread t has the vectors of eight t, t + 256, ... and adds their squares one after the other
+    (a square of two bfloat16 is exact, so a fused multiply-add rounds as the sum does); the lanes of a warp and then the warps as
+    trees."""
+    rows, width = x.shape
+    f = torch.zeros(rows, 8192)
+    f[:, :width] = x.float()
+    f = f.view(rows, 4, 256, 8)
+    sq = torch.zeros(rows, 256)
+    for i in range(4):
+        for k in range(8):
+            sq = sq + f[:, i, :, k] * f[:, i, :, k]
+    sq = sq.view(rows, 8, 32)
+    for half in (16, 8, 4, 2, 1):
+        sq = sq[..., :half] + sq[..., half:2 * half]
+    sq = sq[..., 0]
+    for half in (4, 2, 1):
+        sq = sq[..., :half] + sq[..., half:2 * half]
+    scale = 1.0 / torch.sqrt(sq / width + eps)
+    return ((x.float() * scale).bfloat16().float() * w.float()).bfloat16()
+
+
+@pytest.mark.parametrize("width", [96, 264, 1024, 1032, 2048, 4096, 8192])
+@pytest.mark.parametrize("weight_dtype", [torch.bfloat16, torch.float32])
+def test_the_sum_of_a_row_has_one_order(width, weight_dtype):
+    """Whoever takes a row, a warp or a block, in whatever company: the same bits."""
+    from qwen_inference_lab_b200.kernels import ops
+    generator = torch.Generator().manual_seed(width + 1)
+    x = torch.randn(601, width, generator=generator).bfloat16()
+    w = (1 + 0.1 * torch.randn(width, generator=generator)).to(weight_dtype)
+    wanted = in_the_order_of_256_threads(x, w, 1e-6)
+    for n in (1, 64, 601):
+        assert torch.equal(ops.rmsnorm(x[:n].cuda(), w.cuda(), 1e-6).cpu(), wanted[:n]), n
