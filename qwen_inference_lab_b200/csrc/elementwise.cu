@@ -92,9 +92,8 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const W* __restrict__ we
 
 // bfloat16 rows of up to 256 * 8 * RMS_VPT elements: the whole row sits in registers, every load is
 // 16 bytes wide and issued before the first use, so a row costs one memory round trip, not one per element.
-// TPR threads take a row: 256 of them, or a warp one of up to 1024, which needs no barrier, and a block of a step of many rows
-// eight of those (2920 rows of 1024: 7.9 -> 4.0 us).  128 threads a row of 4096 instead of 256: 2048 rows 9.6 -> 9.1 us, but 64 rows
-// 3.0 -> 3.8, which is what a decode step has.
+// TPR threads take a row: 256 of them, or, in a step of many rows of up to 1024, a warp, eight rows a block and no barrier.
+// 128 threads a row of 4096 instead of 256: 2048 rows 9.6 -> 9.1 us, but 64 rows 3.0 -> 3.8, which is what a decode step has.
 #define RMS_VPT 4
 template <typename W, int TPR>
 __global__ void __launch_bounds__(256)
@@ -104,7 +103,7 @@ rmsnorm_bf16x8_kernel(const bf16* __restrict__ x, const W* __restrict__ weight, 
     qil_wait_for_producer();
     qil_release_consumer();
     static_assert(RMS_VPT == 4 && (TPR == 32 || TPR == 256), "the sum's order below");
-    const int tid = threadIdx.x % TPR, r = blockIdx.x * (blockDim.x / TPR) + threadIdx.x / TPR;
+    const int tid = threadIdx.x % TPR, r = blockIdx.x * (256 / TPR) + threadIdx.x / TPR;
     const bool live = r < n_rows;                 // uniform over a row's threads
     const int src_row = !live ? 0 : rows ? rows[r] : r;
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)src_row * width);
@@ -199,14 +198,14 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const float* __restrict__ weight
     }
 }
 
+// A warp a row pays once the blocks of 256 threads come in more than one round of four an SM.  Rows of 1024, us as blocks / as
+// warps: 1 row 1.36 / 1.76, 64 1.54 / 2.00, 296 1.70 / 2.11, 512 2.33 / 2.26, 593 2.29 / 2.25, 1024 3.11 / 2.33, 2920 6.43 / 2.75.
 template <typename W>
 static void rmsnorm_bf16x8(const bf16* x, const W* weight, const int* rows, bf16* out, int n_rows, int width, float eps, cudaStream_t stream) {
-    auto launch = [&](auto kernel, int tpr) {
-        const int per_block = n_rows > 4 * 148 ? 256 / tpr : 1;       // few rows: a block each, on as many SMs
-        qil_launch_chained(kernel, dim3((n_rows + per_block - 1) / per_block), dim3(tpr * per_block), 0, stream, x, weight, rows, out, n_rows, width, eps);
-    };
-    if (width <= 32 * 8 * RMS_VPT) launch(rmsnorm_bf16x8_kernel<W, 32>, 32);
-    else launch(rmsnorm_bf16x8_kernel<W, 256>, 256);
+    if (width <= 32 * 8 * RMS_VPT && n_rows > 4 * 148)
+        qil_launch_chained(rmsnorm_bf16x8_kernel<W, 32>, dim3((n_rows + 7) / 8), dim3(256), 0, stream, x, weight, rows, out, n_rows, width, eps);
+    else
+        qil_launch_chained(rmsnorm_bf16x8_kernel<W, 256>, dim3(n_rows), dim3(256), 0, stream, x, weight, rows, out, n_rows, width, eps);
 }
 
 extern "C" int qil_rmsnorm(const void* x, const void* weight, const int* rows, void* out,
