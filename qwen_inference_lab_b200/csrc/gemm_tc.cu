@@ -508,7 +508,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // Epilogue: a lane holds a feature, memory wants a token's features side by side.  Two groups of four warps take 32 columns
 // in turn: the warps leave their lanes' float32 sums in the group's staging buffer, then take its rows (a token's 128
 // features; of the q/k/v projection a whole head), four features a lane.  Tensor memory is free for the next tile once
-// it is staged.  Barriers and bounded waits are those of the kernel above.
+// it is staged.  Barriers and bounded waits are those of the kernel above; a group's four warps meet at a barrier of their own,
+// which has no limit, so behind each bounded wait they go on together or leave together.
 #define TE_STAGES 6
 #define TE_W_BYTES (128 * TC_BK * 2)
 #define TE_STAGE_BYTES (2 * TE_W_BYTES)          // and up to 128 tokens
@@ -563,6 +564,15 @@ __device__ __forceinline__ uint2 te_qkv_values(const float4& f, const bf16* norm
 
 // The four warps of an epilogue group meet.
 __device__ __forceinline__ void te_group_sync(int group) { asm volatile("bar.sync %0, 128;\n" ::"r"(group + 1) : "memory"); }
+// The same, and true if all of them come with `ok`: one whose wait ran out takes the other three along, who would otherwise
+// meet without it for good.
+__device__ __forceinline__ bool te_group_agrees(int group, bool ok) {
+    unsigned all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+                 "bar.red.and.pred p, %1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(all) : "r"(group + 1), "r"((unsigned)ok) : "memory");
+    return all != 0;
+}
 
 // The rows of a staged chunk that one of the group's four warps takes: tokens m0 + i of i = part, part + 4, ... < rows, the 128
 // features from n0 on.
@@ -778,11 +788,11 @@ gemm_tc_even_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         qil_wait_for_producer();
         int acc = 0;
         unsigned acc_phase = 0;
-        bool ok = true;
-        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+        for (int tile = pair; tile < n_tiles; tile += n_pairs) {
             const int m0 = (tile % tiles_m) * nt, n0 = (tile / tiles_m) * 256 + (int)rank * 128;
-            if (ok && !mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; }
-            ok = __all_sync(0xffffffffu, ok);
+            const bool ok = warp_mbar_wait(&sh->acc_full[acc], acc_phase);
+            if (!ok && lane == 0) atomicExch(error_word, 5);
+            if (!te_group_agrees(group, ok)) break;      // nothing of this tile is stored
             tc_fence_after();
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * 256;
             for (int c0 = group * TE_CHUNK; c0 < nt; c0 += 2 * TE_CHUNK) {
@@ -793,7 +803,7 @@ gemm_tc_even_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&sh->acc_empty[acc]), 0));
                 }
-                te_group_sync(group);                    // the rows of the chunk before have been read
+                if (c0 >= 2 * TE_CHUNK) te_group_sync(group);      // the rows of the chunk before have been read
 #pragma unroll
                 for (int i = 0; i < 32; ++i) staged[i * 128 + quarter * 32 + lane] = v[i];
                 te_group_sync(group);
