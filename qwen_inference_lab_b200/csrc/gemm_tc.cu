@@ -725,23 +725,14 @@ gemm_tc_even_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         __syncwarp();
         const unsigned full_of_first = uniform(map_to_rank(smem_u32(sh->full), 0));
         const unsigned stage_bytes = 2 * (TE_W_BYTES + nt * TC_BK);            // both blocks' weights and tokens
-        // the ring's first round: weights, which no kernel writes, before the kernel before this one has ended
-        const int first = pair < n_tiles ? (k_blocks < TE_STAGES ? k_blocks : TE_STAGES) : 0;
-        const int first_n = pair / tiles_m * 256 + (int)rank * 128, first_m = pair % tiles_m * nt + (int)rank * (nt / 2);
-        for (int s = 0; s < first; ++s) {
-            mbar_arrive_expect_tx(&sh->full[s], stage_bytes, leader && rank == 0);
-            tma_load_2d_pair(tiles + s * TE_STAGE_BYTES, &map_w, full_of_first + s * 8, s * TC_BK, first_n, leader);
-        }
-        qil_wait_for_producer();
+        qil_wait_for_producer();     // the weights too: a caller's weight may be what the kernel before wrote
         qil_release_consumer();      // the block holds its tensor memory
-        for (int s = 0; s < first; ++s)
-            tma_load_2d_pair(tiles + s * TE_STAGE_BYTES + TE_W_BYTES, &map_x, full_of_first + s * 8, s * TC_BK, first_m, leader);
-        int stage = first == TE_STAGES ? 0 : first;
-        unsigned phase = first == TE_STAGES ? 1 : 0;
+        int stage = 0;
+        unsigned phase = 0;
         bool ok = true;
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const int m0 = tile % tiles_m * nt + (int)rank * (nt / 2), n0 = tile / tiles_m * 256 + (int)rank * 128;
-            for (int kb = tile == pair ? first : 0; kb < k_blocks; ++kb) {
+            for (int kb = 0; kb < k_blocks; ++kb) {
                 if (!warp_mbar_wait(&sh->empty[stage], phase ^ 1)) { if (leader) atomicExch(error_word, 1); ok = false; break; }
                 mbar_arrive_expect_tx(&sh->full[stage], stage_bytes, leader && rank == 0);
                 unsigned char* to = tiles + stage * TE_STAGE_BYTES;

@@ -6,7 +6,7 @@ from pathlib import Path
 import pytest
 
 SOURCE = (Path(__file__).resolve().parent.parent / "qwen_inference_lab_b200" / "csrc" / "gemm_tc.cu").read_text()
-KERNELS = ("gemm_tc_kernel", "gemm_tc_pair_kernel", "gemm_tc_rows_kernel")
+KERNELS = ("gemm_tc_kernel", "gemm_tc_pair_kernel", "gemm_tc_even_kernel", "gemm_tc_rows_kernel")
 
 
 def block(text, at):
@@ -20,8 +20,8 @@ def block(text, at):
     raise AssertionError("unbalanced braces")
 
 
-@pytest.mark.parametrize("kernel", KERNELS)
-def test_every_role_waits_for_the_kernel_before_ahead_of_its_first_bounded_wait(kernel):
+def roles_of(kernel):
+    """The text of the kernel's three roles: loads, MMAs, epilogue."""
     source = re.sub(r"//[^\n]*", "", SOURCE)
     definition = re.search(r"__global__[^;{]*?\b%s\(" % kernel, source)
     assert re.search(r"qil_launch_(chained|clusters)\(%s\b" % kernel, source)
@@ -34,7 +34,22 @@ def test_every_role_waits_for_the_kernel_before_ahead_of_its_first_bounded_wait(
         if not follows:
             break
         at = end
-    assert len(roles) == 3                                 # loads, MMAs, epilogue
-    for role in roles:
+    assert len(roles) == 3
+    return roles
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_every_role_waits_for_the_kernel_before_ahead_of_its_first_bounded_wait(kernel):
+    for role in roles_of(kernel):
         assert "mbar_wait(" in role
         assert role.split("mbar_wait(")[0].count("qil_wait_for_producer();") == 1, role[:200]
+
+
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_what_is_copied_ahead_of_the_wait(kernel):
+    """The tile kernels take any caller's matrices, the output of the kernel before among them; the streaming one asks for its
+    weights first and says so."""
+    ahead, after = roles_of(kernel)[0].split("qil_wait_for_producer();")
+    copied = re.findall(r"tma_load_2d\w*\([^;]*?&(map_\w+)", ahead)
+    assert copied == (["map_w"] if kernel == "gemm_tc_rows_kernel" else [])
+    assert "&map_w" in after

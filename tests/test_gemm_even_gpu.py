@@ -77,3 +77,18 @@ def test_the_rule_takes_ragged_portions_and_leaves_whole_ones(monkeypatch):
         got = gemm_tc.gemm_tc(a, w)
         assert bool(((got.double() - wanted).abs() <= 2.0 ** -8 * 1.01 * wanted.abs() + 2100 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t())).all())
     gemm_tc.check()
+
+
+@pytest.mark.parametrize("m,n,k,tokens", [(300, 2048, 1024, 160), (521, 4096, 2048, 0)])
+def test_a_weight_that_the_kernel_before_has_just_written(m, n, k, tokens):
+    """The norm lets the next kernel begin before it has written its rows."""
+    from qwen_inference_lab_b200.kernels import gemm_tc, ops
+    a, source, gain = draw(m, k), draw(n, k, seed=1), draw(k, seed=2)
+    w = ops.rmsnorm(source, gain, 1e-6)
+    torch.cuda.synchronize()
+    wanted = gemm_tc.gemm_tc(a, w, tile_tokens=tokens)
+    for _ in range(20):
+        w.zero_()
+        ops.rmsnorm(source, gain, 1e-6, out=w)
+        assert torch.equal(gemm_tc.gemm_tc(a, w, tile_tokens=tokens), wanted)
+    gemm_tc.check()
