@@ -514,7 +514,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #define TE_W_BYTES (128 * TC_BK * 2)
 #define TE_STAGE_BYTES (2 * TE_W_BYTES)          // and up to 128 tokens
 #define TE_CHUNK 32                              // tokens a group stages at a time
-#define TE_STAGING_BYTES (TE_CHUNK * 128 * 4)
+#define TE_ROW 132                               // floats a staged token: eight rows side by side are in eight different groups of banks
+#define TE_STAGING_BYTES (TE_CHUNK * TE_ROW * 4)
 
 struct TcEvenShared {
     unsigned long long full[TE_STAGES];
@@ -525,16 +526,32 @@ struct TcEvenShared {
     unsigned pad;
 };
 
+// The factor that norms a staged token's head: the squares of the product's bfloat16 values one after the other, as
+// tc_store_qkv_head adds them, so that a token's bits do not depend on the kernel that its step's size picks.
+__device__ __forceinline__ float te_norm_scale(const float* row, const bf16* __restrict__ bias, float eps) {
+    float sq = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < 128; c += 4) {
+        float4 f = *reinterpret_cast<const float4*>(row + c);
+        if (bias != nullptr) {
+            const uint2 raw = *reinterpret_cast<const uint2*>(bias + c);
+            const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+            f.x += x.x; f.y += x.y; f.z += y.x; f.w += y.y;
+        }
+        const float2 a = __bfloat1622float2(__floats2bfloat162_rn(f.x, f.y)), b = __bfloat1622float2(__floats2bfloat162_rn(f.z, f.w));
+        sq = fmaf(b.y, b.y, fmaf(b.x, b.x, fmaf(a.y, a.y, fmaf(a.x, a.x, sq))));
+    }
+    return rsqrtf(sq / 128.0f + eps);
+}
+
 // One token's head of the q/k/v projection, four values a lane (`f`: the product, with its bias): the arithmetic and the
-// rounding points of tc_store_qkv_head, the sum of squares as a tree over the lanes.  cf, sf: the lane's cosines and sines.
-__device__ __forceinline__ uint2 te_qkv_values(const float4& f, const bf16* norm_w, bool rotate, const float4& cf, const float4& sf,
-                                               float eps, int lane) {
+// rounding points of tc_store_qkv_head.  cf, sf: the lane's cosines and sines.
+__device__ __forceinline__ uint2 te_qkv_values(const float4& f, const bf16* norm_w, float scale, bool rotate, const float4& cf, const float4& sf,
+                                               int lane) {
     typedef __nv_bfloat162 bf2;
     bf2 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
     if (norm_w != nullptr) {
         const float2 a = __bfloat1622float2(lo), b = __bfloat1622float2(hi);
-        const float sq = warp_sum(fmaf(b.y, b.y, fmaf(b.x, b.x, fmaf(a.y, a.y, a.x * a.x))));
-        const float scale = rsqrtf(sq / 128.0f + eps);
         const uint2 w = *reinterpret_cast<const uint2*>(norm_w + lane * 4);
         lo = __hmul2_rn(__floats2bfloat162_rn(a.x * scale, a.y * scale), *reinterpret_cast<const bf2*>(&w.x));
         hi = __hmul2_rn(__floats2bfloat162_rn(b.x * scale, b.y * scale), *reinterpret_cast<const bf2*>(&w.y));
@@ -574,8 +591,8 @@ __device__ __forceinline__ bool te_group_agrees(int group, bool ok) {
     return all != 0;
 }
 
-// The rows of a staged chunk that one of the group's four warps takes: tokens m0 + i of i = part, part + 4, ... < rows, the 128
-// features from n0 on.
+// The rows of a staged chunk that one of the group's four warps takes: tokens m0 + i of i = part, part + 4, ... < rows (of the q/k/v
+// projection eight side by side), the 128 features from n0 on.
 __device__ __forceinline__ void te_store_rows(const float* staged, int part, int rows, int m0, int n0, int N, int silu_pairs,
                                               const bf16* __restrict__ bias, const bf16* residual, bf16* out, const TcQkvTail& tail, int lane) {
     constexpr int R = TE_CHUNK / 4;
@@ -586,8 +603,8 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
 #pragma unroll
         for (int r = 0; r < R; r += 2) {
             const int i = part + 4 * (r + (lane >> 4));
-            const float4 g = *reinterpret_cast<const float4*>(staged + i * 128 + col);
-            const float4 u = *reinterpret_cast<const float4*>(staged + i * 128 + col + 8);
+            const float4 g = *reinterpret_cast<const float4*>(staged + i * TE_ROW + col);
+            const float4 u = *reinterpret_cast<const float4*>(staged + i * TE_ROW + col + 8);
             if (i >= rows || n0 + col >= N) continue;
             const float gate[4] = {g.x, g.y, g.z, g.w}, up[4] = {u.x, u.y, u.z, u.w};
             uint2 packed;
@@ -611,13 +628,13 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
         b = make_float4(x.x, x.y, y.x, y.y);
     }
     if (tail.q_out != nullptr) {
-        // The 128 features are one whole head, and every lane takes part in its sums.  What a row's place and rotation need is
-        // asked for once a chunk, a row a lane, and for four rows at a time: these are trips to L2, one after the other.
+        // The 128 features are one whole head.  What a row's norm, place and rotation need is found once a chunk, a row a lane, and
+        // asked for four rows at a time: these are trips to L2, one after the other.
         const int head = n0 / 128;
         const bool is_q = head < tail.n_q_heads, is_k = !is_q && head < tail.n_q_heads + tail.n_kv_heads;
         const bf16* norm_w = is_q ? tail.q_norm : (is_k ? tail.k_norm : nullptr);
         const bool rotate = (is_q || is_k) && tail.rope != nullptr;
-        const int mine = part + 4 * (lane & (R - 1));
+        const int mine = part * R + (lane & (R - 1));
         int pos_of_lane = 0, page_of_lane = -1;
         if (mine < rows) {
             pos_of_lane = tail.positions[m0 + mine];
@@ -625,6 +642,7 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
             if (!is_q && pos_of_lane >= 0 && index < tail.table_stride)
                 page_of_lane = tail.block_table[(size_t)tail.token_row[m0 + mine] * tail.table_stride + index];
         }
+        const float scale_of_lane = norm_w != nullptr ? te_norm_scale(staged + mine * TE_ROW, bias ? bias + n0 : nullptr, tail.eps) : 1.f;
 #pragma unroll
         for (int r0 = 0; r0 < R; r0 += 4) {
             float4 f[4], cf[4], sf[4];
@@ -633,9 +651,9 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
             for (int u = 0; u < 4; ++u) {
                 pos[u] = __shfl_sync(0xffffffffu, pos_of_lane, r0 + u);
                 const int row = (pos[u] >= tail.rope_rows && tail.rope_rows > 0) ? tail.rope_rows - 1 : pos[u];
-                f[u] = *reinterpret_cast<const float4*>(staged + (part + 4 * (r0 + u)) * 128 + lane * 4);
+                f[u] = *reinterpret_cast<const float4*>(staged + (part * R + r0 + u) * TE_ROW + lane * 4);
                 cf[u] = sf[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (rotate && part + 4 * (r0 + u) < rows) {
+                if (rotate && part * R + r0 + u < rows) {
                     const float* cs = tail.rope + (size_t)row * 128 + (lane & 15) * 4;
                     cf[u] = *reinterpret_cast<const float4*>(cs);
                     sf[u] = *reinterpret_cast<const float4*>(cs + 64);
@@ -643,9 +661,10 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int i = part + 4 * (r0 + u), page = __shfl_sync(0xffffffffu, page_of_lane, r0 + u);
+                const int i = part * R + r0 + u, page = __shfl_sync(0xffffffffu, page_of_lane, r0 + u);
+                const float scale = __shfl_sync(0xffffffffu, scale_of_lane, r0 + u);
                 f[u].x += b.x; f[u].y += b.y; f[u].z += b.z; f[u].w += b.w;
-                const uint2 values = te_qkv_values(f[u], norm_w, rotate, cf[u], sf[u], tail.eps, lane);
+                const uint2 values = te_qkv_values(f[u], norm_w, scale, rotate, cf[u], sf[u], lane);
                 if (i >= rows) continue;
                 bf16* dst;
                 if (is_q) {
@@ -671,7 +690,7 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
     for (int r = 0; r < R; ++r) {
         const int i = part + 4 * r;
         if (i >= rows) break;
-        float4 f = *reinterpret_cast<const float4*>(staged + i * 128 + lane * 4);
+        float4 f = *reinterpret_cast<const float4*>(staged + i * TE_ROW + lane * 4);
         f.x += b.x; f.y += b.y; f.z += b.z; f.w += b.w;
         if (residual != nullptr) {
             const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&held[r].x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&held[r].y));
@@ -796,7 +815,7 @@ gemm_tc_even_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 }
                 if (c0 >= 2 * TE_CHUNK) te_group_sync(group);      // the rows of the chunk before have been read
 #pragma unroll
-                for (int i = 0; i < 32; ++i) staged[i * 128 + quarter * 32 + lane] = v[i];
+                for (int i = 0; i < 32; ++i) staged[i * TE_ROW + quarter * 32 + lane] = v[i];
                 te_group_sync(group);
                 const int rows = min(min(TE_CHUNK, nt - c0), M - m0 - c0);
                 te_store_rows(staged, quarter, rows, m0 + c0, n0, N, silu_pairs, bias, residual, out, tail, lane);

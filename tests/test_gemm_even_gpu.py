@@ -36,9 +36,11 @@ def silu_apart(gemm_tc, a, w, tokens):
 
 
 @pytest.mark.parametrize("m,n_q,n_kv,page,bias,norms,rope", [(300, 3, 1, 8, True, True, True), (521, 4, 2, 16, False, True, True),
-                                                             (260, 2, 0, 16, False, False, False)])
+                                                             (260, 2, 0, 16, False, False, False), (200, 4, 2, 8, True, True, True),
+                                                             (700, 32, 8, 16, False, True, True)])
 def test_the_tail_of_the_projection(m, n_q, n_kv, page, bias, norms, rope):
-    """Against the kernel with one token a lane: the sums of squares come in another order, so a normed value may round the other way."""
+    """The bits of the kernels with one token a lane, which take these as the rule has it: a token's queries and keys do not depend
+    on the tiles that a step's size picks."""
     from qwen_inference_lab_b200.kernels import gemm_tc
     from qwen_inference_lab_b200.parts.rotary import rotary_table
     heads, k = n_q + 2 * n_kv, 256
@@ -60,11 +62,7 @@ def test_the_tail_of_the_projection(m, n_q, n_kv, page, bias, norms, rope):
         results.append((q, pages))
     for q, pages in results[1:]:
         for got, wanted in ((q, results[0][0]), (pages, results[0][1])):
-            assert torch.equal(got == 7.0, wanted == 7.0) or not norms
-            difference = (got.double() - wanted.double()).abs()
-            assert float((difference > 0).double().mean()) < 0.02
-            # one step of bfloat16 in the normed value, and the rotation's three roundings on top, of values up to the row's largest
-            assert float(difference.max()) <= 4 * 2.0 ** -7 * float(wanted.double().abs().max())
+            assert torch.equal(got, wanted)
 
 
 def test_the_rule_takes_ragged_portions_and_leaves_whole_ones(monkeypatch):
