@@ -526,20 +526,29 @@ struct TcEvenShared {
     unsigned pad;
 };
 
-// The factor that norms a staged token's head: the squares of the product's bfloat16 values one after the other, as
-// tc_store_qkv_head adds them, so that a token's bits do not depend on the kernel that its step's size picks.
-__device__ __forceinline__ float te_norm_scale(const float* row, const bf16* __restrict__ bias, float eps) {
-    float sq = 0.f;
-#pragma unroll 8
-    for (int c = 0; c < 128; c += 4) {
-        float4 f = *reinterpret_cast<const float4*>(row + c);
+// The factors that norm the heads of eight staged tokens, lane & 7 of them this lane's: the squares of the product's bfloat16
+// values one after the other, as tc_store_qkv_head adds them, so that a token's bits do not depend on the kernel that its
+// step's size picks.  Lanes of one token square a quarter of the features each; the sum goes through them in their order.
+__device__ __forceinline__ float te_norm_scale(const float* row, const bf16* __restrict__ bias, float eps, int lane) {
+    const int first = lane >> 3 << 5;
+    float v[32];
+#pragma unroll
+    for (int c = 0; c < 32; c += 4) {
+        float4 f = *reinterpret_cast<const float4*>(row + first + c);
         if (bias != nullptr) {
-            const uint2 raw = *reinterpret_cast<const uint2*>(bias + c);
+            const uint2 raw = *reinterpret_cast<const uint2*>(bias + first + c);
             const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
             f.x += x.x; f.y += x.y; f.z += y.x; f.w += y.y;
         }
         const float2 a = __bfloat1622float2(__floats2bfloat162_rn(f.x, f.y)), b = __bfloat1622float2(__floats2bfloat162_rn(f.z, f.w));
-        sq = fmaf(b.y, b.y, fmaf(b.x, b.x, fmaf(a.y, a.y, fmaf(a.x, a.x, sq))));
+        v[c] = a.x; v[c + 1] = a.y; v[c + 2] = b.x; v[c + 3] = b.y;
+    }
+    float sq = 0.f;
+#pragma unroll
+    for (int turn = 0; turn < 4; ++turn) {
+#pragma unroll
+        for (int c = 0; c < 32; ++c) sq = fmaf(v[c], v[c], sq);
+        sq = __shfl_sync(0xffffffffu, sq, turn * 8 + (lane & 7));          // those whose turn it was
     }
     return rsqrtf(sq / 128.0f + eps);
 }
@@ -628,8 +637,8 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
         b = make_float4(x.x, x.y, y.x, y.y);
     }
     if (tail.q_out != nullptr) {
-        // The 128 features are one whole head.  What a row's norm, place and rotation need is found once a chunk, a row a lane, and
-        // asked for four rows at a time: these are trips to L2, one after the other.
+        // The 128 features are one whole head.  A row's place is asked for by a lane of its own, and all rows' rotations before the
+        // sums of squares, whose chain is as long as those trips to L2.
         const int head = n0 / 128;
         const bool is_q = head < tail.n_q_heads, is_k = !is_q && head < tail.n_q_heads + tail.n_kv_heads;
         const bf16* norm_w = is_q ? tail.q_norm : (is_k ? tail.k_norm : nullptr);
@@ -642,40 +651,37 @@ __device__ __forceinline__ void te_store_rows(const float* staged, int part, int
             if (!is_q && pos_of_lane >= 0 && index < tail.table_stride)
                 page_of_lane = tail.block_table[(size_t)tail.token_row[m0 + mine] * tail.table_stride + index];
         }
-        const float scale_of_lane = norm_w != nullptr ? te_norm_scale(staged + mine * TE_ROW, bias ? bias + n0 : nullptr, tail.eps) : 1.f;
+        float4 cf[R], sf[R];
+        int pos[R];
 #pragma unroll
-        for (int r0 = 0; r0 < R; r0 += 4) {
-            float4 f[4], cf[4], sf[4];
-            int pos[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                pos[u] = __shfl_sync(0xffffffffu, pos_of_lane, r0 + u);
-                const int row = (pos[u] >= tail.rope_rows && tail.rope_rows > 0) ? tail.rope_rows - 1 : pos[u];
-                f[u] = *reinterpret_cast<const float4*>(staged + (part * R + r0 + u) * TE_ROW + lane * 4);
-                cf[u] = sf[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (rotate && part * R + r0 + u < rows) {
-                    const float* cs = tail.rope + (size_t)row * 128 + (lane & 15) * 4;
-                    cf[u] = *reinterpret_cast<const float4*>(cs);
-                    sf[u] = *reinterpret_cast<const float4*>(cs + 64);
-                }
+        for (int r = 0; r < R; ++r) {
+            pos[r] = __shfl_sync(0xffffffffu, pos_of_lane, r);
+            const int row = (pos[r] >= tail.rope_rows && tail.rope_rows > 0) ? tail.rope_rows - 1 : pos[r];
+            cf[r] = sf[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (rotate && part * R + r < rows) {
+                const float* cs = tail.rope + (size_t)row * 128 + (lane & 15) * 4;
+                cf[r] = *reinterpret_cast<const float4*>(cs);
+                sf[r] = *reinterpret_cast<const float4*>(cs + 64);
             }
+        }
+        const float scale_of_lane = norm_w != nullptr ? te_norm_scale(staged + mine * TE_ROW, bias ? bias + n0 : nullptr, tail.eps, lane) : 1.f;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = part * R + r0 + u, page = __shfl_sync(0xffffffffu, page_of_lane, r0 + u);
-                const float scale = __shfl_sync(0xffffffffu, scale_of_lane, r0 + u);
-                f[u].x += b.x; f[u].y += b.y; f[u].z += b.z; f[u].w += b.w;
-                const uint2 values = te_qkv_values(f[u], norm_w, scale, rotate, cf[u], sf[u], lane);
-                if (i >= rows) continue;
-                bf16* dst;
-                if (is_q) {
-                    dst = tail.q_out + ((size_t)(m0 + i) * tail.n_q_heads + head) * 128;
-                } else {
-                    if (page < 0 || page >= tail.num_pages) continue;        // never write outside the pool
-                    const int kv_head = is_k ? head - tail.n_q_heads : head - tail.n_q_heads - tail.n_kv_heads;
-                    dst = tail.pages + ((((size_t)page * 2 + (is_k ? 0 : 1)) * tail.n_kv_heads + kv_head) * tail.page_size + pos[u] % tail.page_size) * 128;
-                }
-                *reinterpret_cast<uint2*>(dst + lane * 4) = values;
+        for (int r = 0; r < R; ++r) {
+            const int i = part * R + r, page = __shfl_sync(0xffffffffu, page_of_lane, r);
+            const float scale = __shfl_sync(0xffffffffu, scale_of_lane, r);
+            float4 f = *reinterpret_cast<const float4*>(staged + i * TE_ROW + lane * 4);
+            f.x += b.x; f.y += b.y; f.z += b.z; f.w += b.w;
+            const uint2 values = te_qkv_values(f, norm_w, scale, rotate, cf[r], sf[r], lane);
+            if (i >= rows) continue;
+            bf16* dst;
+            if (is_q) {
+                dst = tail.q_out + ((size_t)(m0 + i) * tail.n_q_heads + head) * 128;
+            } else {
+                if (page < 0 || page >= tail.num_pages) continue;        // never write outside the pool
+                const int kv_head = is_k ? head - tail.n_q_heads : head - tail.n_q_heads - tail.n_kv_heads;
+                dst = tail.pages + ((((size_t)page * 2 + (is_k ? 0 : 1)) * tail.n_kv_heads + kv_head) * tail.page_size + pos[r] % tail.page_size) * 128;
             }
+            *reinterpret_cast<uint2*>(dst + lane * 4) = values;
         }
         return;
     }
