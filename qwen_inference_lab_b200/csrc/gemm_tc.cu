@@ -1139,13 +1139,21 @@ static int tokens_a_tile(int M, int tiles_n, int pairs, long long* cost) {
 }
 
 // Does the even kernel take the product?  Where even tiles make its waves a tenth cheaper than those of 256 (from 256
-// tokens on, pairs of blocks) or 128 tokens (one block).  Its epilogue goes through shared memory and is the slower one: a long K
-// hides it, and a single wave of tiles has it only once; that of q/k/v (`tail`) wants the long K.
-// Measured, us (the other kernels / this one, weights from memory):
-//   gate/up of 24576 x 4096: 129 tokens 60 / 48, 300 69 / 58, 521 94 / 75, 1021 137 / 136 (not taken), 2048 256 / 256 (not taken)
-//   gate/up of 6144 x 1024:  129 tokens 11.4 / 8.3, 300 12.0 / 9.9, 521 12.5 / 12.1, 1021 16.6 / 16.9 (not taken), 2048 22.6 / 26.7 (not taken)
-//   q/k/v of 6144 x 4096:    521 tokens 34.1 / 31.0, 700 34.3 / 39.7 (not taken), 1021 51.3 / 45.1, 1500 55 / 61 (not taken)
-//   q/k/v of 4096 x 1024:    521 tokens 17.5 / 17.6, 700 18.1 / 19.0, 1021 18.2 / 24.9 (none taken)
+// tokens on, pairs of blocks) or 128 tokens (one block), and K is long enough to hide an epilogue that goes through shared
+// memory and grows with a tile's tokens.  A single wave of tiles has it once, that of q/k/v (`tail`) is the longer one.  The lines
+// lie where every product measured on the even side is at least as fast.
+// Measured, us (the other kernels / this one at the tokens a tile in brackets, weights from memory):
+//   gate/up of 24576 x 4096: 129 tokens 64 / 48, 300 73 / 58, 521 102 / 79, 2048 256 / 256 (waves no cheaper: not taken)
+//   gate/up in two waves:    12288 x 2048 at 300 tokens 25.6 / 19.5, 521 28.2 / 23.8; K below 2048 not taken (9216 x 1536 at 521 20.9 / 17.7,
+//                            but 9216 x 1024 at 700 17.1 / 18.1)
+//   gate/up in one wave:     6144 x 1024 at 129 11.1 / 8.3, 300 12.0 / 9.9, 521 [176] 12.4 / 12.1, 560 [192] 12.4 / 12.5 (not taken);
+//                            4608 x 768 at 480 [128] 10.2 / 9.3, 700 [176] 10.8 / 11.2 (not taken); 4608 x 256 at 300 [80] 7.2 / 6.4, 480 [128]
+//                            7.3 / 7.4 (not taken); 6144 x 96 at 128 [48] 6.1 / 5.5, 255 [96] 6.2 / 6.5 (not taken)
+//   q/k/v in one wave:       6144 x 4096 at 521 33.2 / 31.3; 4096 x 2048 at 512 [128] 21.9 / 18.1, 600 [160] 22.3 / 22.0, 700 [176]
+//                            22.8 / 23.0 (not taken); 6144 x 2560 at 512 [176] 25.7 / 25.1, 560 [192] 25.4 / 25.9 (not taken)
+//   q/k/v in more:           6144 x 4096 at 776 [144] 50 / 41, 1021 [176] 51 / 46; 5120 x 3072 at 850 [128] 35.7 / 31.2, 1021 [160] 36.1 / 36.7
+//                            (not taken); 4096 x 3584 at 1350 [160] 40.2 / 39.1, 1500 [176] 40.5 / 41.7 (not taken); 4096 x 2048 at 1200 [144]
+//                            28.1 / 31.9 (not taken)
 static int even_tokens(int M, int N, int K, bool tail, int pairs, int sm_count) {
     const int tiles_n = (N + 255) / 256;
     long long cost;
@@ -1154,8 +1162,15 @@ static int even_tokens(int M, int N, int K, bool tail, int pairs, int sm_count) 
     const long long others = M >= 256 ? (long long)((M + 255) / 256) * tiles_n : (long long)((M + TC_BM - 1) / TC_BM) * tiles_n;
     const int at_a_time = M >= 256 ? pairs : sm_count;
     const long long other_cost = (others + at_a_time - 1) / at_a_time * 128;
-    const bool hidden = K >= 2048 || (tiles <= pairs && !tail);
+    const bool one_wave = tiles <= pairs;
+    const bool hidden = !tail ? K >= 2048 || (one_wave && nt <= 48 + K / 8)
+                              : one_wave ? K >= 2048 && nt <= 96 + K / 32 : nt <= K / 16 - 64;
     return hidden && 10 * cost <= 9 * other_cost ? nt : 0;
+}
+
+// The rule by itself: the tokens a tile, 0 for another kernel.
+extern "C" int qil_gemm_tc_even_tokens(int M, int N, int K, int tail, int pairs, int sm_count) {
+    return even_tokens(M, N, K, tail != 0, pairs, sm_count);
 }
 
 // nt: tokens a tile of the even kernel (0: as even_tokens says, which may be another kernel).
