@@ -21,18 +21,44 @@ def test_tiles_of_any_number_of_tokens(m, n, k, tokens):
     out = residual.clone()
     gemm_tc.gemm_tc(a, w, bias=bias, residual=out, out=out, tile_tokens=tokens)
     assert bool(((out.double() - wanted).abs() <= bound).all())
-    if n % 16 == 0:
-        assert torch.equal(gemm_tc.gemm_tc(a, w, silu_pairs=True, tile_tokens=tokens), silu_apart(gemm_tc, a, w, tokens))
     gemm_tc.check()
 
 
-def silu_apart(gemm_tc, a, w, tokens):
-    from qwen_inference_lab_b200.kernels import ops
-    hidden = ops.silu_mul(gemm_tc.gemm_tc(a, w, tile_tokens=tokens), pairs8=True)
-    # the fused form divides approximately before it rounds to bfloat16
-    fused = gemm_tc.gemm_tc(a, w, silu_pairs=True, tile_tokens=tokens)
-    assert bool(((fused.double() - hidden.double()).abs() <= 2.0 ** -6 * hidden.double().abs()).all())
-    return fused
+@pytest.mark.parametrize("tokens", [16, 48, 176, 256])
+@pytest.mark.parametrize("m,n,k", [(1, 16, 8), (31, 144, 72), (177, 272, 200), (521, 640, 448), (1030, 1040, 384)])
+def test_gate_and_up_in_one(m, n, k, tokens):
+    from qwen_inference_lab_b200.kernels import gemm_tc, ops
+    a, w = draw(m, k), draw(n, k, seed=1, scale=2 * k ** -0.5)
+    fused = gemm_tc.gemm_tc(a, w, silu_pairs=True, tile_tokens=tokens).double()
+    gate, up = (a.double() @ w.double().t()).view(m, n // 16, 2, 8).unbind(2)
+    slack = (k + 4) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()).view(m, n // 16, 2, 8)
+    # the sums in float32, then rounded to bfloat16 (half a step of 8 bits); silu's slope is at most 1.1
+    half = 2.0 ** -8 * 1.01
+    off_gate, off_up = half * gate.abs() + slack[:, :, 0], half * up.abs() + slack[:, :, 1]
+    silu = torch.nn.functional.silu(gate)
+    off_silu = 1.1 * off_gate
+    off_silu += half * (silu.abs() + off_silu)
+    wanted = silu * up
+    off = off_silu * (up.abs() + off_up) + silu.abs() * off_up
+    off += half * (wanted.abs() + off)
+    assert bool(((fused.view_as(wanted) - wanted).abs() <= off).all())
+    # and beside the same product with its activation apart, which does not divide approximately
+    hidden = ops.silu_mul(gemm_tc.gemm_tc(a, w, tile_tokens=tokens), pairs8=True).double()
+    assert bool(((fused - hidden).abs() <= 2.0 ** -6 * hidden.abs()).all())
+    gemm_tc.check()
+
+
+@pytest.mark.parametrize("m,n,k", [(255, 9216, 96), (1021, 6144, 1024), (700, 4608, 768)])
+def test_gate_and_up_have_the_bits_of_the_other_kernels(m, n, k):
+    """Products that the rule leaves to the tile and pair kernels."""
+    from qwen_inference_lab_b200.kernels import gemm_tc
+    from tests.test_even_rule import taken
+    a, w = draw(m, k), draw(n, k, seed=1, scale=k ** -0.5)
+    assert taken(m, n, k) == 0
+    wanted = gemm_tc.gemm_tc(a, w, silu_pairs=True)
+    for tokens in (16, 96, 176, 256):
+        assert torch.equal(gemm_tc.gemm_tc(a, w, silu_pairs=True, tile_tokens=tokens), wanted), tokens
+    gemm_tc.check()
 
 
 @pytest.mark.parametrize("m,n_q,n_kv,page,bias,norms,rope", [(300, 3, 1, 8, True, True, True), (521, 4, 2, 16, False, True, True),
@@ -65,8 +91,8 @@ def test_the_tail_of_the_projection(m, n_q, n_kv, page, bias, norms, rope):
             assert torch.equal(got, wanted)
 
 
-def test_the_rule_takes_ragged_portions_and_leaves_whole_ones(monkeypatch):
-    """The same product with and without the rule: the kernels agree to the last rounding."""
+def test_products_whose_tiles_the_rule_chooses():
+    """Whole and ragged numbers of tokens against 64 bits; which kernel takes them is `test_even_rule`'s."""
     from qwen_inference_lab_b200.kernels import gemm_tc
     w = draw(2048, 2048, scale=2048 ** -0.5)
     for m in (129, 255, 256, 257, 300, 512, 521):
