@@ -341,7 +341,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int buf = j & 1, stage = j % AT_STAGES;
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j);
-            if (!mbar_wait(&sh->s_full[buf], (j >> 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 21); ok = false; break; }
+            if (!warp_mbar_wait(&sh->s_full[buf], (j >> 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 21); ok = false; break; }
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j + 1);
             tc_fence_after();
             float s[AT_N];
@@ -422,7 +422,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 // second MMA waits for this warp.  After it, it could also be a phase behind (another warp still at its
                 // rescale of the tile before), which the parity of the last wait below cannot tell from done: so the
                 // last tile waits here whether it rescales or not.  Its second MMA follows the awaited one anyway.
-                if (!mbar_wait(&sh->pv_done, (j - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 22); ok = false; break; }
+                if (!warp_mbar_wait(&sh->pv_done, (j - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 22); ok = false; break; }
                 tc_fence_after();
             }
             if (rescale) {
@@ -441,7 +441,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             // on the last tile, value rows past the last visible key may hold anything (unwritten slots):
             // zero them so that 0 * garbage cannot become NaN; they are this thread's key row
             if (j == n_tiles - 1) {
-                if (!mbar_wait(&sh->v_full[stage], (j / AT_STAGES) & 1)) { if (lane == 0) atomicExch(p.error_word, 23); ok = false; break; }
+                if (!warp_mbar_wait(&sh->v_full[stage], (j / AT_STAGES) & 1)) { if (lane == 0) atomicExch(p.error_word, 23); ok = false; break; }
                 if (row < AT_N && key0 + row > hi) {
                     unsigned char* v_row = sV + stage * AT_VTILE + row * 128;
 #pragma unroll
@@ -468,7 +468,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             if (warp == 2 && lane == 0) AT_STAMP(2, 6 * j + 5);
         }
         if (ok) {
-            if (!mbar_wait(&sh->pv_done, (n_tiles - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 24); ok = false; }
+            if (!warp_mbar_wait(&sh->pv_done, (n_tiles - 1) & 1)) { if (lane == 0) atomicExch(p.error_word, 24); ok = false; }
         }
         if (ok) {
             tc_fence_after();

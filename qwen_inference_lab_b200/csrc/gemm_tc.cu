@@ -300,7 +300,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         bool ok = true;
         for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * TC_BN;
-            if (!mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; break; }
+            if (!warp_mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; break; }
             tc_fence_after();
             const int m = m0 + quarter * 32 + lane;
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * TC_BN + half;
@@ -475,7 +475,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         bool ok = true;
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const int m0 = (tile % tiles_m) * 256 + (int)rank * 128, n0 = (tile / tiles_m) * TC_BN;
-            if (!mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; break; }
+            if (!warp_mbar_wait(&sh->acc_full[acc], acc_phase)) { if (lane == 0) atomicExch(error_word, 5); ok = false; break; }
             tc_fence_after();
             const int m = m0 + quarter * 32 + lane;
             const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)acc * TC_BN + half;
@@ -966,7 +966,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     } else {
         const int quarter = warp & 3;
         qil_wait_for_producer();
-        if (mbar_wait(&sh->acc_full, 0)) {          // every stage has been read: the ring is free
+        if (warp_mbar_wait(&sh->acc_full, 0)) {          // every stage has been read: the ring is free
             tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < ROWS / 32; ++c) {

@@ -50,7 +50,8 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     return true;
 }
 
-// The same for a whole warp, which goes on together.
+// The same for a whole warp, which goes on or gives up together: lanes that left by themselves would be missing from the
+// warp-wide instructions that follow.
 __device__ __forceinline__ bool warp_mbar_wait(unsigned long long* bar, unsigned parity) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
 }

@@ -1,10 +1,14 @@
-"""The even kernel's epilogue: four warps that meet at a barrier without a limit, each behind a bounded wait of its own."""
+"""Behind a bounded wait goes on together what meets again without a limit: the lanes of a warp, and the four warps of an even
+kernel's epilogue group."""
 import itertools
 import re
+from pathlib import Path
 
 import pytest
 
-from tests.test_chained_waits import SOURCE, block
+from tests.test_chained_waits import KERNELS, SOURCE, block, roles_of
+
+ATTENTION = (Path(__file__).resolve().parent.parent / "qwen_inference_lab_b200" / "csrc" / "attention_tc.cu").read_text()
 
 
 def outcome(passes, chunks, agree):
@@ -58,3 +62,15 @@ def test_the_kernel_votes_before_it_reads_or_stores():
         assert name not in before and name in after
     assert "mbar_wait(" not in after
     assert re.search(r"bar\.red\.and\.pred p, %1, 128, q;", SOURCE)
+
+
+@pytest.mark.parametrize("kernel", KERNELS + ("attn_tc_kernel",))
+def test_the_lanes_of_a_warp_go_on_together(kernel):
+    """A lane that gave up by itself would be missing from the warp's reads of tensor memory."""
+    if kernel == "attn_tc_kernel":
+        source = re.sub(r"//[^\n]*", "", ATTENTION)
+        role, _ = block(source, source.index("} else if (warp < AT_VALUE_WARP) {") + 2)
+    else:
+        role = roles_of(kernel)[2]
+    waits = re.findall(r"\w*mbar_wait\(", role)
+    assert waits and set(waits) == {"warp_mbar_wait("}
