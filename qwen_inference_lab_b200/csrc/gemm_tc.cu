@@ -3,13 +3,13 @@
 // portions (M from a few dozen to thousands of tokens).
 //
 // Blackwell-native structure, one persistent block per SM, 320 threads:
-//   warp 0      one thread issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a
-//               128 x 64 tile of A and a 256 x 64 tile of W per stage into a 4-stage ring and
-//               arms the stage's mbarrier with the byte count;
-//   warp 1      one thread issues tcgen05.mma (128 x 256 x 16, operands from shared memory
-//               through matrix descriptors, accumulator in tensor memory) four times per stage,
-//               then tcgen05.commit, which frees the stage when the MMAs have read it; the warp
-//               also allocates and frees the 512 columns of tensor memory;
+//   warp 0      walks the stages of a 4-stage ring; its elected lane arms a stage's mbarrier with the
+//               byte count and issues the TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a
+//               128 x 64 tile of A and a 256 x 64 tile of W;
+//   warp 1      walks them behind it; its elected lane issues tcgen05.mma (128 x 256 x 16, operands from
+//               shared memory through matrix descriptors, accumulator in tensor memory) four times per
+//               stage, then tcgen05.commit, which frees the stage when the MMAs have read it; the warp
+//               also allocates and frees the 512 columns of tensor memory (why the warps walk along: tcgen05.cuh);
 //   warps 2-9   read the finished accumulator with tcgen05.ld (each warp its quarter of the 128
 //               lanes and one half of the columns), apply the epilogue and store bfloat16; meanwhile warp 1 already fills
 //               the other half of tensor memory with the next tile.
@@ -1298,11 +1298,12 @@ static int launch_rows(const CUtensorMap& map_x, const CUtensorMap& map_w, const
     QIL_CHECK_LAUNCH();
 }
 
-// M <= 128 rows; the rest as qil_gemm_tc.  (Products without silu_pairs come with up to 32 rows unless the caller's line is raised:
-// from 40 on the library's are faster in a step.)  Measured, us for a tile's K cut into 1 / 2 / 4 / 8 at 32 rows, weights from
-// memory: 6144 x 1024 9.3 / 6.5 / 8.0 / 14.9, 4096 x 4096 23.1 / 14.2 / 12.1 / 11.8, 6144 x 4096 23.5 / 15.3 / 14.2 / 20.1,
-// 1024 x 3072 18.2 / 10.9 / 7.7 / 6.8, 24576 x 4096 37.3 / 42.0 / 46 / 64: what a block adds up grows with the rows and the
-// cluster, so K is cut while a block keeps six stages and the blocks are at most four thirds of the SMs.
+// M <= 128 rows; the rest as qil_gemm_tc.  (The rows that come without silu_pairs end at a line of the caller's.)  w must be written
+// before the kernel before this one begins: it is read while that one may still run.  Measured, us for a tile's K cut into
+// 1 / 2 / 4 / 8 at 32 rows, weights from memory: 6144 x 1024 7.2 / 5.8 / 5.8 / 11.4, 4096 x 4096 16.4 / 10.9 / 9.8 / 9.6, 6144 x 4096
+// 17.2 / 12.4 / 11.7 / 16.2, 1024 x 3072 12.4 / 7.6 / 5.7 / 5.7, 24576 x 4096 35.2 / 37.5 / 40.6 / 51.7; at 64 rows 6144 x 1024
+// 8.9 / 6.3 / 7.3 / 14.9, 4096 x 4096 20.7 / 12.9 / 10.4 / 11.7, 24576 x 4096 37.4 / 41.6 / 46.5 / 65.9: what a block adds up grows with the
+// rows and the cluster, so K is cut while a block keeps six stages and the blocks are at most four thirds of the SMs.
 extern "C" int qil_gemm_tc_rows(const void* a, const void* w, const void* bias, const void* residual, void* out,
                                 int M, int N, int K, int silu_pairs, int sm_count, int* error_word, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;

@@ -93,7 +93,8 @@ def rows_usable(a, weight, silu_pairs=False, residual=None, out=None) -> bool:
 
 
 def gemm_rows(a, weight, bias=None, residual=None, out=None, silu_pairs=False):
-    """``gemm_tc`` for at most 128 rows: the weights are streamed once, K cut over clusters of blocks."""
+    """``gemm_tc`` for at most 128 rows: the weights are streamed once, K cut over clusters of blocks.  ``weight`` is read while
+    the kernel before this one may still run, so it must not be what that kernel writes (``gemm_tc`` takes such a one)."""
     _need(a, "a", torch.bfloat16, 2); _need(weight, "weight", torch.bfloat16, 2)
     m, k = a.shape
     n = weight.shape[0]

@@ -254,6 +254,7 @@ def gemm_small_m(a, weight, bias=None, residual=None, out=None, out_float32=Fals
                  norm_weight=None, norm_eps=0.0, rows_per_block=None, col_scale=None, activation=None):
     """out = a @ weight.T (+ bias) (+ residual) for a decode step's few rows, streaming the weight once.
 
+    ``weight`` and ``norm_weight`` are read while the kernel before this one may still run: they must not be what it writes.
     a bfloat16 [M <= 16, K]; weight bfloat16 [N, K].  ``out_float32`` returns float32 (the LM head).
     ``silu_pairs``: weight rows are groups of [8 gate, 8 up]; returns silu(gate) * up, bfloat16 [M, N/2].
     ``residual`` may be ``out`` itself.  With ``norm_weight`` (bfloat16 [K]) the kernel first applies

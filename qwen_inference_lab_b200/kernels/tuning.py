@@ -33,21 +33,27 @@ SMALL_M_WIDE_MAX_ELEMENTS = _tuned("SMALL_M_WIDE_MAX_ELEMENTS", 1 << 28)
 #: take): the streaming one up to the limits below, from there on the tile kernel.
 TILE_KERNEL_MIN_ROWS = _tuned("TILE_KERNEL_MIN_ROWS", 17)
 #: Up to this many rows the streaming tcgen05 kernel (``gemm_tc.gemm_rows``) takes the gate/up product of a matrix of at
-#: least 148 tiles of 128 features, and any number up to its 128 of a smaller one (24576 x 4096 against the tile kernel:
-#: 38.9 / 41.0 us at 64 rows, 42.9 / 40.3 at 128; 6144 x 1024: 8.2 / 12.3 and 10.0 / 12.3).  Where K is cut over a cluster the
+#: least 148 tiles of 128 features, and any number up to its 128 of a smaller one (us, alone, against the tile kernels, the even
+#: tiles among them: 24576 x 4096 37.0 / 39.9 at 33 rows, 38.1 / 40.1 at 64, 41.0 / 40.3 at 96, 42.4 / 40.4 at 128; 6144 x 1024
+#: 5.9 / 7.9, 6.8 / 7.9, 8.4 / 8.0, 9.0 / 8.5: the line of the smaller one was drawn before there were even tiles).  Where K is cut
+#: over a cluster the
 #: sums come in another order than the tile kernel's; against 64 bits both are as far off (12 shapes of K 96 to 25600, 17 to 128
 #: rows, 3 seeds each: relative errors of 3.50e-3 to 3.65e-3, ratio 0.996 to 1.003 either way).
 ROWS_PAIRS_MAX = _tuned("ROWS_PAIRS_MAX", 64)
-#: ... and every other product instead of the library's.  Alone the two are even (4096 x 4096 12.1 / 11.1 us at 32 rows, 4096 x
-#: 12288 22.9 / 23.5, 1024 x 2048 6.5 / 7.2); in a chain this one's start is hidden.  A recorded step of the 28-layer 1024-wide
-#: model with both, with gate/up alone and without: 1231 / 1252 / 1385 us at 17 rows, 1291 / 1391 / 1510 at 24, 1383 / 1419 / 1538 at
-#: 32, 1440 / 1418 / 1457 at 40; of the 36-layer 4096-wide one 3780 / 3871 / 3976, 3851 / 3951 / 4057, 4001 / 4022 / 4122, 4140 / 4073 / 4142.
+#: ... and every other product instead of the library's.  Alone the two are even (us, this one / the library's: 4096 x 4096
+#: 10.3 / 9.4 at 32 rows, 4096 x 12288 20.5 / 21.4, 1024 x 3072 5.9 / 7.4, 4096 x 1024 5.1 / 4.5); in a chain this one's start is
+#: hidden.  A recorded step of the 28-layer 1024-wide model behind 500 cached tokens with both, with gate/up alone and without (us):
+#: 1170 / 1358 / 1323 at 17 rows, 1284 / 1433 / 1471 at 24, 1367 / 1384 / 1491 at 32, 1447 / 1540 / 1566 at 40, 1544 / 1593 / 1619 at 48,
+#: 1976 / 2033 / 2063 at 64; of the 36-layer 4096-wide one 3662 / 3918 / 4054, 3813 / 4019 / 4158, 3992 / 4074 / 4201, 4155 / 4247 / 4331,
+#: 4218 / 4324 / 4404, 4885 / 4844 / 4917.  So the line could lie at 48 now; it is where it was before the kernel's issue got cheaper
+#: (it lost at 40 then), and a step's bits with it.
 #: (The kernel itself takes up to 128 rows here too, for whoever raises the line.)  Against 64 bits a plain product is as far
 #: off as the library's (1.66e-3), one with a residual less (1.66e-3 against 2.15e-3: one rounding instead of two).
 ROWS_PLAIN_MAX = _tuned("ROWS_PLAIN_MAX", 32)
-#: From this many rows on the q/k/v product runs on the tcgen05 kernels with its tail fused; below, the pair
-#: kernel has too few 256 x 256 tiles for the SM pairs and the library product plus the tail kernel win
-#: (6144 x 4096 at 2048 rows: 86 us against 75 + 24 us; at 256 rows the library wins).
+#: From this many rows on the q/k/v product runs on the tcgen05 kernels with its tail fused; below, the library's product
+#: and the tail kernel.  us, fused / apart: 6144 x 4096 at 256 rows 24 / 20, 512 30 / 28, 700 33 / 34, 1021 46 / 46, 2048 77 / 90,
+#: 2920 105 / 138; 4096 x 1024 at 512 17.2 / 12.0, 700 17.8 / 14.2, 1021 17.8 / 17.8, 2048 28.6 / 29.9, 2920 33.9 / 40.0.  (Kernels alone,
+#: recorded: in a step that is not, as prompts are, the host launches one kernel less.)
 QKV_TAIL_MIN_ROWS = _tuned("QKV_TAIL_MIN_ROWS", 512)
 #: The single-token attention's cost model, in units of the time a block takes to stream one 64-key tile:
 #: a block's start-up (its description, page ids and first tile arrive one after the other) and what each
